@@ -101,8 +101,8 @@ int Plan::init(int n_, long long nrhs_, const double co[7], int prec, int sweeps
   if (rc) return rc;
   rc = cuda_status(cudaMemcpy(d_lw, host.data(), sizeof(double) * 2 * (size_t)n, cudaMemcpyHostToDevice),
                    "cudaMemcpy(factor tables)");
-  if (rc) return rc;
-  return NTK_OK;
+  if (rc || precision != NTK_FP64) return rc;
+  return chunk.init(n, lu_l.data(), lu_u.data(), host.data() + n);
 }
 
 Plan::~Plan() {
@@ -123,12 +123,13 @@ int Plan::g_table(double s, const double** out) {
     set_error("more than 16 distinct RHS scales used with one plan");
     return NTK_ERR_UNSUPPORTED;
   }
-  std::vector<double> g(n);
+  std::vector<double> g(n + chunk.g_elems);
   for (int i = 0; i < n; ++i) g[i] = s / lu_u[i];
+  chunk.g_rows(g.data(), g.data() + n);
   double* d = nullptr;
-  int rc = cuda_status(cudaMalloc(&d, sizeof(double) * (size_t)n), "cudaMalloc(g table)");
+  int rc = cuda_status(cudaMalloc(&d, sizeof(double) * g.size()), "cudaMalloc(g table)");
   if (rc) return rc;
-  rc = cuda_status(cudaMemcpy(d, g.data(), sizeof(double) * (size_t)n, cudaMemcpyHostToDevice), "cudaMemcpy(g)");
+  rc = cuda_status(cudaMemcpy(d, g.data(), sizeof(double) * g.size(), cudaMemcpyHostToDevice), "cudaMemcpy(g)");
   if (rc) {
     cudaFree(d);
     return rc;
@@ -158,6 +159,9 @@ int Plan::run(const double* in, double* out, const Batch& b, RhsParams rp, doubl
     t.w = d_lw + n;
     rc = g_table(s, &t.g);
     if (rc) return rc;
+    int S = 0;
+    if (const ChunkF64::Cfg* cfg = chunk_f64_pick(chunk, b, rp.kind, &S))
+      return launch_chunk_f64(chunk, *cfg, S, in, out, b, rp, t, t.g + n, stream);
     return launch_thomas_f64(in, out, n, b, rp, t, tune_f64_threads, stream, tune_f64_x_variant);
   }
   return run_refine(in, out, b, rp, s, stream);

@@ -1,0 +1,474 @@
+// ntk_chunk_f64.cu -- FP64 solves of few systems, T threads per system.
+//
+// One thread per system (ntk_solve_f64.cu) needs the fewest FP64
+// instructions, but a 256 x 256 field has 256 systems and an ADI sweep of a
+// 2048 x 2048 one 2046: 8 and 64 warps for 152 SMs, each walking 2 n
+// dependent rows through global memory.  Here a CTA keeps S whole systems in
+// shared memory and gives every system T threads of C consecutive rows:
+//   forward   y_i = d_i - l_i y_{i-1} over the chunk from zero, in place;
+//             the chunks' carries are an exact affine scan over the T chunk
+//             ends (log2 T steps through shared memory, the products of the
+//             multipliers tabulated on the host: one FMA a step)
+//   backward  y_i = y'_i + phi_i y_{s-1}, x_i = g_i y_i - (c_i / u_i) x_{i+1}
+//             from zero, then the same scan from the other end
+//   last      x_i = x'_i + psi_i x_{e+1}, stored
+// (phi, psi: the responses of a chunk's sweeps to the carry entering it, as
+// in ntk_adi_f64.cu.)  Nothing is truncated, so any matrix that factors is
+// served, at 5 FP64 instructions a row (+1 for the compact difference)
+// against 3 (+1): the FP64 pipe (one warp instruction per ~73 clocks and
+// sub-partition) bounds both kernels, and this one wins where one thread per
+// system leaves the pipe idle (chunk_f64_pick).
+// Rows stay in shared memory between the sweeps, not in registers, so a
+// chunk may be long: the scans' 2 log2 T instructions a thread are spread
+// over C rows.  C is odd, so the threads of a half-warp, C doubles apart in a
+// dense row, touch 16 different bank pairs; strided systems lie side by side,
+// S to a row, and a half-warp reads whole row segments.
+// Threads whose chunks see bitwise equal factors share one table (the head's
+// few chunks before the pivots reach their fixed point, the interior, the
+// tail), so the factors stay in L1.
+// Measured, one thread per system against this kernel: 2046 systems of 2048
+// rows 754 -> 67 us (FP64 pipe alone: 42 us), compact derivative of a 256 x
+// 256 field 97 -> 11.5 us (most of it the call).
+// A system with a value that is not finite, or that overflows on the way, is
+// solved again row by row from its input, so that inf and nan spread exactly
+// as in the one-thread sweeps.
+#include "ntk_chunk_f64.h"
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "ntk_device.cuh"
+
+namespace ntk {
+
+namespace {
+
+constexpr int RB = 4;  // rows per batch of a sweep: their loads are issued ahead of the dependent FMAs
+
+struct ChunkParams {
+  int n, S, T, C, CP, P, steps, shift;  // shift: log2 S (strided) or log2 T (contiguous)
+  const double* tab;   // [ncls][4][CP]: -l, phi, -w, psi
+  const double* g;     // [ncls][CP]
+  const double* scan;  // [2][steps][T]
+  const int* cls;      // [T]
+  TablesF64 plain;
+};
+
+__device__ __forceinline__ bool finite(double x) { return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u; }
+
+// One system row by row from global memory, the forward values parked in out
+// (which may be in: the compact difference keeps its neighbours in registers).
+template <int RHS>
+__device__ __noinline__ void plain_system(const double* in, double* out, long long base, long long es, int n,
+                                          long long s, const RhsParams& rp, const TablesF64& t) {
+  const double* a = in + base;
+  double* o = out + base;
+  double y = 0.0, fm = 0.0, fc = a[0], d0 = fc, dn = 0.0;
+  if (RHS == RHS_COMPACT) {
+    const double* e = a + (long long)(n - 1) * es;
+    d0 = rp.sigma0 * ((-5.0 * a[0] + 4.0 * a[es]) + a[2 * es]);
+    dn = rp.sigmaN * ((-5.0 * e[0] + 4.0 * e[-es]) + e[-2 * es]);
+  }
+  if (RHS == RHS_CROSS) {
+    d0 = rp.bnd[s * rp.bnd_ss];
+    dn = rp.bnd[s * rp.bnd_ss + (long long)(n - 1) * rp.bnd_es];
+  }
+  for (int i = 0; i < n; ++i) {
+    const double* q = a + (long long)i * es;
+    double d;
+    if (RHS == RHS_COMPACT) {
+      const double fn = i < n - 1 ? q[es] : 0.0;
+      d = fn - fm;
+      fm = fc;
+      fc = fn;
+    } else if (RHS == RHS_CROSS) {
+      d = i == 0 || i == n - 1 ? 0.0
+          : rp.center == 0.0   ? -q[-rp.cs] - q[rp.cs]
+                               : fma(rp.top, q[rp.cs], fma(rp.center, q[0], rp.bottom * q[-rp.cs]));
+    } else {
+      d = q[0];
+    }
+    if (RHS != RHS_IDENTITY && i == n - 1) d = dn;
+    if (RHS != RHS_IDENTITY && i == 0) d = d0;
+    y = i == 0 ? d : fma(-t.l[i], y, d);
+    o[(long long)i * es] = y;
+  }
+  double x = t.g[n - 1] * y;
+  o[(long long)(n - 1) * es] = x;
+  for (int i = n - 2; i >= 0; --i) {
+    x = fma(-t.w[i], x, t.g[i] * o[(long long)i * es]);
+    o[(long long)i * es] = x;
+  }
+}
+
+template <int RHS, bool STRIDED>
+__global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double* out, Batch b,
+                                                        const __grid_constant__ RhsParams rp,
+                                                        const __grid_constant__ ChunkParams c) {
+  extern __shared__ __align__(16) double smem[];
+  const int nt = c.S * c.T;
+  double* tile = smem;
+  double* ex = smem + (STRIDED ? c.S * c.n : c.S * c.P);  // [2][nt]
+  const int tid = threadIdx.x;
+  const int s = STRIDED ? tid & (c.S - 1) : tid >> c.shift;
+  const int t = STRIDED ? tid >> c.shift : tid & (c.T - 1);
+  const int xs = STRIDED ? c.S : 1;  // one chunk on in ex
+  const int rs = STRIDED ? c.S : 1;  // one row on in the tile
+  const long long sys = (long long)blockIdx.x * c.S + s;
+  const bool on = sys < b.nsys;
+  const long long base = !on ? 0 : b.ni >= b.nsys ? sys * b.is : (sys / b.ni) * b.os + (sys % b.ni) * b.is;
+  double* col = tile + (STRIDED ? s : s * c.P);  // row r of this system: col[r * rs]
+
+  // ---- stage the system's rows (the ADI stencil is formed on the way) ----
+  if (on) {
+    const double* src = in + base;
+    if (RHS == RHS_CROSS) {
+#pragma unroll 4
+      for (int r = t; r < c.n; r += c.T) {
+        const double* q = src + (long long)r * b.es;
+        double v;
+        if (r == 0 || r == c.n - 1) v = rp.bnd[sys * rp.bnd_ss + (long long)r * rp.bnd_es];
+        else if (rp.center == 0.0) v = -q[-rp.cs] - q[rp.cs];
+        else v = fma(rp.top, q[rp.cs], fma(rp.center, q[0], rp.bottom * q[-rp.cs]));
+        col[r * rs] = v;
+      }
+    } else {
+#pragma unroll 4
+      for (int r = t; r < c.n; r += c.T) cp_async8(col + r * rs, src + (long long)r * b.es, 8u);
+      cp_async_wait_all();
+    }
+  }
+  __syncthreads();
+
+  const int r0 = t * c.C;
+  const int len = on ? max(0, min(c.C, c.n - r0)) : 0;
+  double* row = col + r0 * rs;  // row r0 + k: row[k * rs]
+  const int cls = __ldg(c.cls + t);
+  const double* ml = c.tab + (size_t)cls * 4 * c.CP;
+  const double* phi = ml + c.CP;
+  const double* mw = phi + c.CP;
+  const double* psi = mw + c.CP;
+  const double* g = c.g + (size_t)cls * c.CP;
+
+  // ---- forward over the chunk from zero ----
+  double y = 0.0;
+  {
+    double fm = 0.0, fr = 0.0, bh = 0.0, bt = 0.0;
+    if (RHS == RHS_COMPACT) {
+      if (len > 0) {
+        fm = r0 > 0 ? row[-rs] : 0.0;
+        fr = r0 + len < c.n ? row[len * rs] : 0.0;
+        if (r0 == 0) bh = rp.sigma0 * ((-5.0 * col[0] + 4.0 * col[rs]) + col[2 * rs]);
+        if (r0 + len == c.n) {
+          const double* e = col + (c.n - 1) * rs;
+          bt = rp.sigmaN * ((-5.0 * e[0] + 4.0 * e[-rs]) + e[-2 * rs]);
+        }
+      }
+      __syncthreads();  // the neighbours' edge rows are read before any row is overwritten
+    }
+    double v[RB];
+#pragma unroll
+    for (int q = 0; q < RB; ++q) v[q] = q < len ? row[q * rs] : 0.0;
+    for (int k = 0; k < len; k += RB) {
+      double nx[RB], m[RB];
+#pragma unroll
+      for (int q = 0; q < RB; ++q) {
+        nx[q] = k + RB + q < len ? row[(k + RB + q) * rs] : 0.0;
+        m[q] = __ldg(ml + k + q);
+      }
+#pragma unroll
+      for (int q = 0; q < RB; ++q) {
+        if (k + q < len) {
+          double d = v[q];
+          if (RHS == RHS_COMPACT) {
+            const double fn = k + q + 1 == len ? fr : q + 1 < RB ? v[(q + 1) % RB] : nx[0];
+            d = fn - fm;
+            fm = v[q];
+            if (r0 + k + q == 0) d = bh;
+            if (r0 + k + q == c.n - 1) d = bt;
+          }
+          y = fma(m[q], y, d);
+          row[(k + q) * rs] = y;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < RB; ++q) v[q] = nx[q];
+    }
+  }
+  // ---- inclusive scan of the chunk ends: y becomes the value of the
+  // chunk's last row with all carries ----
+  int cur = 0;
+  ex[tid] = y;
+  for (int k = 0; k < c.steps; ++k) {
+    const int o = 1 << k;
+    __syncthreads();
+    if (t >= o) y = fma(__ldg(c.scan + k * c.T + t), ex[cur * nt + tid - o * xs], y);
+    cur ^= 1;
+    ex[cur * nt + tid] = y;
+  }
+  __syncthreads();
+  const double cin = t > 0 ? ex[cur * nt + tid - xs] : 0.0;
+
+  // ---- backward over the chunk from zero ----
+  double x = 0.0;
+  {
+    const int k0 = (len - 1) & ~(RB - 1);
+    double v[RB];
+#pragma unroll
+    for (int q = 0; q < RB; ++q) v[q] = len > 0 && k0 + q < len ? row[(k0 + q) * rs] : 0.0;
+    for (int k = k0; k >= 0; k -= RB) {
+      double nx[RB], p[RB], w[RB], gg[RB];
+#pragma unroll
+      for (int q = 0; q < RB; ++q) {
+        nx[q] = k >= RB ? row[(k - RB + q) * rs] : 0.0;
+        p[q] = __ldg(phi + k + q);
+        w[q] = __ldg(mw + k + q);
+        gg[q] = __ldg(g + k + q);
+      }
+#pragma unroll
+      for (int q = RB - 1; q >= 0; --q) {
+        if (k + q < len) {
+          x = fma(w[q], x, gg[q] * fma(p[q], cin, v[q]));
+          row[(k + q) * rs] = x;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < RB; ++q) v[q] = nx[q];
+    }
+  }
+  // ---- the same scan from the other end; the buffer read for cin is left
+  // alone until the first barrier ----
+  cur ^= 1;
+  ex[cur * nt + tid] = x;
+  for (int k = 0; k < c.steps; ++k) {
+    const int o = 1 << k;
+    __syncthreads();
+    if (t + o < c.T) x = fma(__ldg(c.scan + (c.steps + k) * c.T + t), ex[cur * nt + tid + o * xs], x);
+    cur ^= 1;
+    ex[cur * nt + tid] = x;
+  }
+  __syncthreads();
+  const double xin = t < c.T - 1 ? ex[cur * nt + tid + xs] : 0.0;
+  // whatever is not finite anywhere in the system has reached row 0
+  const bool ok = finite(ex[cur * nt + tid - t * xs]);
+
+  // ---- carries into the chunk, results out ----
+  if (STRIDED) {
+    if (on && ok) {
+      double* dst = out + base + (long long)r0 * b.es;
+#pragma unroll 4
+      for (int k = 0; k < len; ++k) dst[(long long)k * b.es] = fma(__ldg(psi + k), xin, row[k * rs]);
+    }
+  } else {
+#pragma unroll 4
+    for (int k = 0; k < len; ++k) row[k] = fma(__ldg(psi + k), xin, row[k]);
+    __syncthreads();
+    if (on && ok) {
+      double* dst = out + base;
+#pragma unroll 4
+      for (int r = t; r < c.n; r += c.T) dst[r] = col[r];
+    }
+  }
+  if (on && !ok && t == 0) plain_system<RHS>(in, out, base, b.es, c.n, sys, rp, c.plain);
+}
+
+// Pitch of a contiguous system in the tile, in doubles: for T < 16 an odd
+// multiple of T, so that the systems of a half-warp lie in different banks.
+int pitch(const ChunkF64::Cfg& cfg, int n) {
+  int P = n;
+  if (cfg.T < 16)
+    while (P % (2 * cfg.T) != cfg.T) ++P;
+  return P;
+}
+size_t smem_bytes(const ChunkF64::Cfg& cfg, int n, int S, bool strided) {
+  const size_t tile = (size_t)S * (strided ? n : pitch(cfg, n));
+  return (tile + 2 * (size_t)S * cfg.T) * sizeof(double);
+}
+
+int log2_of(int v) {
+  int k = 0;
+  while ((1 << k) < v) ++k;
+  return k;
+}
+
+constexpr size_t SMEM_MAX = 220 * 1024;
+constexpr size_t SMEM_SM = 228 * 1024;
+constexpr int SMS = 152;
+constexpr int MAXT = 256;
+
+template <int RHS, bool STRIDED>
+int launch_one(const double* in, double* out, const Batch& b, const RhsParams& rp, const ChunkParams& c, size_t smem,
+               cudaStream_t st) {
+  auto k = chunk_f64_kernel<RHS, STRIDED>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(chunk_f64_kernel)");
+  const long long blocks = (b.nsys + c.S - 1) / c.S;
+  k<<<(unsigned)blocks, c.S * c.T, smem, st>>>(in, out, b, rp, c);
+  return cuda_status(cudaGetLastError(), "chunk_f64_kernel");
+}
+
+}  // namespace
+
+ChunkF64::~ChunkF64() {
+  if (d_tab) cudaFree(d_tab);
+}
+
+int ChunkF64::init(int n_, const double* l, const double* u, const double* w) {
+  n = n_;
+  std::vector<double> tab;
+  for (int T = 4; T <= MAXT; T *= 2) {
+    Cfg f;
+    f.T = T;
+    f.C = ((n + T - 1) / T) | 1;
+    if (f.C < 5 || smem_bytes(f, n, std::max(1, 32 / T), false) > SMEM_MAX) continue;
+    f.CP = (f.C + RB - 1) / RB * RB;
+    f.tab = tab.size();
+    f.g = g_elems;
+    std::vector<double> Phi(T, 0.0), Psi(T, 0.0);
+    std::vector<int> cls(T);
+    for (int t = 0; t < T; ++t) {
+      const int r0 = t * f.C, len = std::max(0, std::min(f.C, n - r0));
+      int id = -1;  // a chunk seen before with bitwise equal factors in all rows
+      for (int j = 0; j < f.ncls && id < 0; ++j) {
+        const int q0 = f.rep[j] * f.C, qlen = std::max(0, std::min(f.C, n - q0));
+        const size_t bytes = sizeof(double) * len;
+        if (qlen == len && (len == 0 || (std::memcmp(l + q0, l + r0, bytes) == 0 &&
+                                         std::memcmp(u + q0, u + r0, bytes) == 0 &&
+                                         std::memcmp(w + q0, w + r0, bytes) == 0)))
+          id = j;
+      }
+      if (id < 0) {
+        id = f.ncls++;
+        f.rep.push_back(t);
+        // its columns; rows past the system's end hold zeros
+        const size_t at = tab.size();
+        tab.resize(at + 4 * (size_t)f.CP, 0.0);
+        double* q = tab.data() + at;
+        double p = 1.0;
+        for (int k = 0; k < len; ++k) {
+          q[k] = -l[r0 + k];
+          p *= -l[r0 + k];
+          q[f.CP + k] = p;
+          q[2 * f.CP + k] = -w[r0 + k];
+        }
+        Phi[t] = len ? p : 0.0;
+        p = 1.0;
+        for (int k = len - 1; k >= 0; --k) {
+          p *= -w[r0 + k];
+          q[3 * f.CP + k] = p;
+        }
+        Psi[t] = len ? p : 0.0;
+      } else {
+        Phi[t] = Phi[f.rep[id]];
+        Psi[t] = Psi[f.rep[id]];
+      }
+      cls[t] = id;
+    }
+    // scan multipliers: step k combines chunk t with the result of chunk
+    // t - 2^k (t + 2^k from the other end)
+    f.scan = tab.size();
+    const int steps = log2_of(T);
+    tab.resize(tab.size() + 2 * (size_t)steps * T, 0.0);
+    double* sf = tab.data() + f.scan;
+    double* sb = sf + (size_t)steps * T;
+    for (int k = 0; k < steps; ++k)
+      for (int t = 0; t < T; ++t) {
+        const int o = 1 << k >> 1;
+        if (k == 0) sf[t] = Phi[t], sb[t] = Psi[t];
+        else {
+          sf[k * T + t] = t >= o ? sf[(k - 1) * T + t] * sf[(k - 1) * T + t - o] : 0.0;
+          sb[k * T + t] = t + o < T ? sb[(k - 1) * T + t] * sb[(k - 1) * T + t + o] : 0.0;
+        }
+      }
+    f.cls = tab.size();
+    tab.resize(tab.size() + (T + 1) / 2, 0.0);
+    std::memcpy(tab.data() + f.cls, cls.data(), sizeof(int) * T);
+    g_elems += (size_t)f.ncls * f.CP;
+    cfgs.push_back(f);
+  }
+  if (cfgs.empty()) return NTK_OK;
+  int rc = cuda_status(cudaMalloc(&d_tab, tab.size() * sizeof(double)), "cudaMalloc(chunk tables)");
+  if (!rc)
+    rc = cuda_status(cudaMemcpy(d_tab, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice),
+                     "cudaMemcpy(chunk tables)");
+  return rc;
+}
+
+void ChunkF64::g_rows(const double* g, double* out) const {
+  for (const Cfg& f : cfgs)
+    for (int j = 0; j < f.ncls; ++j)
+      for (int k = 0; k < f.CP; ++k) {
+        const int r = f.rep[j] * f.C + k;
+        out[f.g + (size_t)j * f.CP + k] = k < f.C && r < n ? g[r] : 0.0;
+      }
+}
+
+// Costs in FP64 warp instructions of one sub-partition (~73 clocks each).
+// Chunks: a CTA's threads run C (5 + extra) row instructions, the two scans
+// and ~14 instructions' worth of staging and barriers; an SM's share of them
+// runs at the pipe's rate plus, once per wave of resident CTAs, the length of
+// one CTA's dependent chain.  One thread per system: n (3 + extra)
+// instructions a warp, times the measured distance from the pipe's rate, which
+// falls with the number of warps that hide each other's loads (a sub-partition
+// needs several; 512 rows, us, thread-per-system against chunks: contiguous
+// 4096 systems 179 : 29, 16384 181 : 104, 65536 362 : 363; strided compact
+// 16384 162 : 124, 49152 251 : 331).
+const ChunkF64::Cfg* chunk_f64_pick(const ChunkF64& c, const Batch& b, int rhs, int* S) {
+  const bool strided = b.es != 1;
+  const int extra = rhs == RHS_COMPACT ? 1 : 0;
+  const ChunkF64::Cfg* best = nullptr;
+  double best_cost = 0.0;
+  for (const ChunkF64::Cfg& f : c.cfgs)
+    for (int s = strided ? 4 : std::max(1, 32 / f.T); s <= 16; s *= 2) {
+      const int nt = s * f.T;
+      const size_t smem = smem_bytes(f, c.n, s, strided);
+      const long long ctas = (b.nsys + s - 1) / s;
+      if (nt < 32 || nt > 512 || smem > SMEM_MAX || ctas > 0x7fffffffLL) continue;
+      const double per_sm = std::ceil((double)ctas / SMS);
+      const double resident = std::min<double>(std::min(32, 2048 / nt), SMEM_SM / (smem + 1024));
+      const double unit = f.C * (5 + extra) + 2 * log2_of(f.T) + 14;
+      const double cost = unit * (per_sm * nt / 128 + std::ceil(per_sm / resident));
+      if (!best || cost < best_cost) {
+        best_cost = cost;
+        best = &f;
+        *S = s;
+      }
+    }
+  const double load = std::ceil((double)((b.nsys + 31) / 32) / (4 * SMS));
+  const double far = strided ? 1.05 + 0.65 / load : 1.15 + 1.9 / load;
+  return best && best_cost < load * c.n * (3 + extra) * far ? best : nullptr;
+}
+
+int launch_chunk_f64(const ChunkF64& cf, const ChunkF64::Cfg& cfg, int S, const double* in, double* out,
+                     const Batch& b, const RhsParams& rp, const TablesF64& t, const double* g, cudaStream_t st) {
+  const bool strided = b.es != 1;
+  ChunkParams c;
+  c.n = cf.n;
+  c.S = S;
+  c.T = cfg.T;
+  c.C = cfg.C;
+  c.CP = cfg.CP;
+  c.P = pitch(cfg, cf.n);
+  c.steps = log2_of(cfg.T);
+  c.shift = strided ? log2_of(S) : c.steps;
+  c.tab = cf.d_tab + cfg.tab;
+  c.g = g + cfg.g;
+  c.scan = cf.d_tab + cfg.scan;
+  c.cls = reinterpret_cast<const int*>(cf.d_tab + cfg.cls);
+  c.plain = t;
+  const size_t smem = smem_bytes(cfg, cf.n, S, strided);
+  switch (rp.kind) {
+    case RHS_COMPACT:
+      return strided ? launch_one<RHS_COMPACT, true>(in, out, b, rp, c, smem, st)
+                     : launch_one<RHS_COMPACT, false>(in, out, b, rp, c, smem, st);
+    case RHS_CROSS:
+      return strided ? launch_one<RHS_CROSS, true>(in, out, b, rp, c, smem, st)
+                     : launch_one<RHS_CROSS, false>(in, out, b, rp, c, smem, st);
+    default:
+      return strided ? launch_one<RHS_IDENTITY, true>(in, out, b, rp, c, smem, st)
+                     : launch_one<RHS_IDENTITY, false>(in, out, b, rp, c, smem, st);
+  }
+}
+
+}  // namespace ntk

@@ -4,6 +4,7 @@
 #include <mutex>
 #include <vector>
 
+#include "ntk_chunk_f64.h"
 #include "ntk_internal.h"
 
 #define NTK_STR2(x) #x
@@ -68,7 +69,8 @@ struct Plan {
   int device = -1;
   std::vector<double> lu_l, lu_u;   // host LU factors (FP64)
   double* d_lw = nullptr;           // device: l[n], w[n]
-  std::map<double, double*> g_by_scale;  // device g = s/u per RHS scale
+  ChunkF64 chunk;                   // NTK_FP64 with few systems: T threads per system
+  std::map<double, double*> g_by_scale;  // device g = s/u per RHS scale: g[n], then chunk's g rows
   RefineState* refine = nullptr;
   LongRefine* long_refine = nullptr;  // FP32 / FP32+refine windows for n > 1024
   SpikeSolver* spike = nullptr;       // n > 1024 where the windows' halos do not decay: exact partitions
