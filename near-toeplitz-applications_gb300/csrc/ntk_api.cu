@@ -123,9 +123,10 @@ int Plan::g_table(double s, const double** out) {
     set_error("more than 16 distinct RHS scales used with one plan");
     return NTK_ERR_UNSUPPORTED;
   }
-  std::vector<double> g(n + chunk.g_elems);
+  const size_t rows = chunk.g_offset(n);
+  std::vector<double> g(rows + chunk.g_elems());
   for (int i = 0; i < n; ++i) g[i] = s / lu_u[i];
-  chunk.g_rows(g.data(), g.data() + n);
+  chunk.g_rows(g.data(), g.data() + rows);
   double* d = nullptr;
   int rc = cuda_status(cudaMalloc(&d, sizeof(double) * g.size()), "cudaMalloc(g table)");
   if (rc) return rc;
@@ -161,7 +162,7 @@ int Plan::run(const double* in, double* out, const Batch& b, RhsParams rp, doubl
     if (rc) return rc;
     int S = 0;
     if (const ChunkF64::Cfg* cfg = chunk_f64_pick(chunk, b, rp.kind, &S))
-      return launch_chunk_f64(chunk, *cfg, S, in, out, b, rp, t, t.g + n, stream);
+      return launch_chunk_f64(chunk, *cfg, S, in, out, b, rp, t, stream);
     return launch_thomas_f64(in, out, n, b, rp, t, tune_f64_threads, stream, tune_f64_x_variant);
   }
   return run_refine(in, out, b, rp, s, stream);

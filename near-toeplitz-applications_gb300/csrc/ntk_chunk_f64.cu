@@ -14,21 +14,23 @@
 //   last      x_i = x'_i + psi_i x_{e+1}, stored
 // (phi, psi: the responses of a chunk's sweeps to the carry entering it, as
 // in ntk_adi_f64.cu.)  Nothing is truncated, so any matrix that factors is
-// served, at 5 FP64 instructions a row (+1 for the compact difference)
+// served, at 5 operations a row (+1 for the compact difference)
 // against 3 (+1): the FP64 pipe (one warp instruction per ~73 clocks and
 // sub-partition) bounds both kernels, and this one wins where one thread per
 // system leaves the pipe idle (chunk_f64_pick).
 // Rows stay in shared memory between the sweeps, not in registers, so a
 // chunk may be long: the scans' 2 log2 T instructions a thread are spread
-// over C rows.  C is odd, so the threads of a half-warp, C doubles apart in a
-// dense row, touch 16 different bank pairs; strided systems lie side by side,
-// S to a row, and a half-warp reads whole row segments.
+// over C rows.  A contiguous system's chunks lie C + 1 doubles apart (odd: the
+// threads of a half-warp touch 16 different bank pairs); strided systems lie
+// side by side, S to a row, and a half-warp reads whole row segments.
+// The scaling g y, off the dependent chain, runs on the integer pipes
+// (ntk_soft_f64.cuh), which leaves 4 (+1) FP64 instructions a row.
 // Threads whose chunks see bitwise equal factors share one table (the head's
 // few chunks before the pivots reach their fixed point, the interior, the
 // tail), so the factors stay in L1.
 // Measured, one thread per system against this kernel: 2046 systems of 2048
-// rows 754 -> 67 us (FP64 pipe alone: 42 us), compact derivative of a 256 x
-// 256 field 97 -> 11.5 us (most of it the call).
+// rows 754 -> 45 us (67 with g y on the FP64 pipe; the pipe alone: 34 us),
+// compact derivative of a 256 x 256 field 97 -> 11.5 us (most of it the call).
 // A system with a value that is not finite, or that overflows on the way, is
 // solved again row by row from its input, so that inf and nan spread exactly
 // as in the one-thread sweeps.
@@ -47,9 +49,11 @@ namespace {
 constexpr int RB = 4;  // rows per batch of a sweep: their loads are issued ahead of the dependent FMAs
 
 struct ChunkParams {
-  int n, S, T, C, CP, P, steps, shift;  // shift: log2 S (strided) or log2 T (contiguous)
-  const double* tab;   // [ncls][4][CP]: -l, phi, -w, psi
-  const double* g;     // [ncls][CP]
+  int n, S, T, C, P, steps, shift;  // P: pitch of a contiguous system; shift: log2 S (strided) or log2 T
+  unsigned invC;       // ceil(2^32 / C): r / C = umulhi(r, invC) for the rows of a system
+  const double* tab;      // [ncls][4][C]: -l, phi, -w, psi
+  const double* g;        // [ncls][C]
+  const SoftFactor* sg;   // the same, prepared
   const double* scan;  // [2][steps][T]
   const int* cls;      // [T]
   TablesF64 plain;
@@ -102,6 +106,11 @@ __device__ __noinline__ void plain_system(const double* in, double* out, long lo
   }
 }
 
+__device__ __forceinline__ SoftFactor load_factor(const SoftFactor* p) {
+  const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+  return SoftFactor{(uint64_t)q.y << 32 | q.x, q.z, q.w};
+}
+
 template <int RHS, bool STRIDED>
 __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double* out, Batch b,
                                                         const __grid_constant__ RhsParams rp,
@@ -118,7 +127,8 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
   const long long sys = (long long)blockIdx.x * c.S + s;
   const bool on = sys < b.nsys;
   const long long base = !on ? 0 : b.ni >= b.nsys ? sys * b.is : (sys / b.ni) * b.os + (sys % b.ni) * b.is;
-  double* col = tile + (STRIDED ? s : s * c.P);  // row r of this system: col[r * rs]
+  double* col = tile + (STRIDED ? s : s * c.P);  // row r of this system: col[slot(r)]
+  auto slot = [&](int r) { return STRIDED ? r * c.S : r + (int)__umulhi((unsigned)r, c.invC); };
 
   // ---- stage the system's rows (the ADI stencil is formed on the way) ----
   if (on) {
@@ -131,11 +141,11 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
         if (r == 0 || r == c.n - 1) v = rp.bnd[sys * rp.bnd_ss + (long long)r * rp.bnd_es];
         else if (rp.center == 0.0) v = -q[-rp.cs] - q[rp.cs];
         else v = fma(rp.top, q[rp.cs], fma(rp.center, q[0], rp.bottom * q[-rp.cs]));
-        col[r * rs] = v;
+        col[slot(r)] = v;
       }
     } else {
 #pragma unroll 4
-      for (int r = t; r < c.n; r += c.T) cp_async8(col + r * rs, src + (long long)r * b.es, 8u);
+      for (int r = t; r < c.n; r += c.T) cp_async8(col + slot(r), src + (long long)r * b.es, 8u);
       cp_async_wait_all();
     }
   }
@@ -143,26 +153,28 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
 
   const int r0 = t * c.C;
   const int len = on ? max(0, min(c.C, c.n - r0)) : 0;
-  double* row = col + r0 * rs;  // row r0 + k: row[k * rs]
+  double* row = col + (STRIDED ? r0 * c.S : t * (c.C + 1));  // row r0 + k: row[k * rs]
   const int cls = __ldg(c.cls + t);
-  const double* ml = c.tab + (size_t)cls * 4 * c.CP;
-  const double* phi = ml + c.CP;
-  const double* mw = phi + c.CP;
-  const double* psi = mw + c.CP;
-  const double* g = c.g + (size_t)cls * c.CP;
+  const double* ml = c.tab + (size_t)cls * 4 * c.C;
+  const double* phi = ml + c.C;
+  const double* mw = phi + c.C;
+  const double* psi = mw + c.C;
+  const double* g = c.g + (size_t)cls * c.C;
+  const SoftFactor* sg = c.sg + (size_t)cls * c.C;
 
   // ---- forward over the chunk from zero ----
   double y = 0.0;
   {
-    double fm = 0.0, fr = 0.0, bh = 0.0, bt = 0.0;
+    // the neighbours' edge rows, and the end rows' one-sided stencils
+    double fm = 0.0, fr = 0.0, be = 0.0;
     if (RHS == RHS_COMPACT) {
       if (len > 0) {
-        fm = r0 > 0 ? row[-rs] : 0.0;
-        fr = r0 + len < c.n ? row[len * rs] : 0.0;
-        if (r0 == 0) bh = rp.sigma0 * ((-5.0 * col[0] + 4.0 * col[rs]) + col[2 * rs]);
-        if (r0 + len == c.n) {
-          const double* e = col + (c.n - 1) * rs;
-          bt = rp.sigmaN * ((-5.0 * e[0] + 4.0 * e[-rs]) + e[-2 * rs]);
+        fm = r0 > 0 ? col[slot(r0 - 1)] : 0.0;
+        fr = r0 + len < c.n ? col[slot(r0 + len)] : 0.0;
+        const bool tail = r0 + len == c.n;
+        if (r0 == 0 || tail) {
+          const int e = tail ? c.n - 1 : 0, d = tail ? -1 : 1;
+          be = one_sided(tail ? rp.sigmaN : rp.sigma0, col[slot(e)], col[slot(e + d)], col[slot(e + 2 * d)]);
         }
       }
       __syncthreads();  // the neighbours' edge rows are read before any row is overwritten
@@ -185,8 +197,7 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
             const double fn = k + q + 1 == len ? fr : q + 1 < RB ? v[(q + 1) % RB] : nx[0];
             d = fn - fm;
             fm = v[q];
-            if (r0 + k + q == 0) d = bh;
-            if (r0 + k + q == c.n - 1) d = bt;
+            if (r0 + k + q == 0 || r0 + k + q == c.n - 1) d = be;
           }
           y = fma(m[q], y, d);
           row[(k + q) * rs] = y;
@@ -218,21 +229,30 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
 #pragma unroll
     for (int q = 0; q < RB; ++q) v[q] = len > 0 && k0 + q < len ? row[(k0 + q) * rs] : 0.0;
     for (int k = k0; k >= 0; k -= RB) {
-      double nx[RB], p[RB], w[RB], gg[RB];
+      double nx[RB], gy[RB];
+      SoftFactor f[RB];
+      bool in_range = true;
 #pragma unroll
       for (int q = 0; q < RB; ++q) {
         nx[q] = k >= RB ? row[(k - RB + q) * rs] : 0.0;
-        p[q] = __ldg(phi + k + q);
-        w[q] = __ldg(mw + k + q);
-        gg[q] = __ldg(g + k + q);
+        f[q] = load_factor(sg + k + q);
       }
 #pragma unroll
-      for (int q = RB - 1; q >= 0; --q) {
+      for (int q = 0; q < RB; ++q) {
+        v[q] = fma(__ldg(phi + k + q), cin, v[q]);
+        in_range = in_range && (k + q >= len || soft_in_range(v[q], f[q]));
+        gy[q] = soft_product(v[q], f[q]);
+      }
+      if (!in_range) {
+#pragma unroll
+        for (int q = 0; q < RB; ++q) gy[q] = rare_mul(v[q], __ldg(g + k + q));
+      }
+#pragma unroll
+      for (int q = RB - 1; q >= 0; --q)
         if (k + q < len) {
-          x = fma(w[q], x, gg[q] * fma(p[q], cin, v[q]));
+          x = fma(__ldg(mw + k + q), x, gy[q]);
           row[(k + q) * rs] = x;
         }
-      }
 #pragma unroll
       for (int q = 0; q < RB; ++q) v[q] = nx[q];
     }
@@ -267,22 +287,17 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
     if (on && ok) {
       double* dst = out + base;
 #pragma unroll 4
-      for (int r = t; r < c.n; r += c.T) dst[r] = col[r];
+      for (int r = t; r < c.n; r += c.T) dst[r] = col[slot(r)];
     }
   }
   if (on && !ok && t == 0) plain_system<RHS>(in, out, base, b.es, c.n, sys, rp, c.plain);
 }
 
-// Pitch of a contiguous system in the tile, in doubles: for T < 16 an odd
-// multiple of T, so that the systems of a half-warp lie in different banks.
-int pitch(const ChunkF64::Cfg& cfg, int n) {
-  int P = n;
-  if (cfg.T < 16)
-    while (P % (2 * cfg.T) != cfg.T) ++P;
-  return P;
-}
+// Pitch of a contiguous system in the tile, in doubles: C + 1, odd, for each
+// chunk.
+int pitch(const ChunkF64::Cfg& cfg) { return cfg.T * (cfg.C + 1); }
 size_t smem_bytes(const ChunkF64::Cfg& cfg, int n, int S, bool strided) {
-  const size_t tile = (size_t)S * (strided ? n : pitch(cfg, n));
+  const size_t tile = (size_t)S * (strided ? n : pitch(cfg));
   return (tile + 2 * (size_t)S * cfg.T) * sizeof(double);
 }
 
@@ -320,11 +335,10 @@ int ChunkF64::init(int n_, const double* l, const double* u, const double* w) {
   for (int T = 4; T <= MAXT; T *= 2) {
     Cfg f;
     f.T = T;
-    f.C = ((n + T - 1) / T) | 1;
-    if (f.C < 5 || smem_bytes(f, n, std::max(1, 32 / T), false) > SMEM_MAX) continue;
-    f.CP = (f.C + RB - 1) / RB * RB;
+    f.C = ((n + T - 1) / T + RB - 1) / RB * RB;
+    if (n < 5 * T || smem_bytes(f, n, std::max(1, 32 / T), false) > SMEM_MAX) continue;
     f.tab = tab.size();
-    f.g = g_elems;
+    f.g = g_count;
     std::vector<double> Phi(T, 0.0), Psi(T, 0.0);
     std::vector<int> cls(T);
     for (int t = 0; t < T; ++t) {
@@ -343,20 +357,20 @@ int ChunkF64::init(int n_, const double* l, const double* u, const double* w) {
         f.rep.push_back(t);
         // its columns; rows past the system's end hold zeros
         const size_t at = tab.size();
-        tab.resize(at + 4 * (size_t)f.CP, 0.0);
+        tab.resize(at + 4 * (size_t)f.C, 0.0);
         double* q = tab.data() + at;
         double p = 1.0;
         for (int k = 0; k < len; ++k) {
           q[k] = -l[r0 + k];
           p *= -l[r0 + k];
-          q[f.CP + k] = p;
-          q[2 * f.CP + k] = -w[r0 + k];
+          q[f.C + k] = p;
+          q[2 * f.C + k] = -w[r0 + k];
         }
         Phi[t] = len ? p : 0.0;
         p = 1.0;
         for (int k = len - 1; k >= 0; --k) {
           p *= -w[r0 + k];
-          q[3 * f.CP + k] = p;
+          q[3 * f.C + k] = p;
         }
         Psi[t] = len ? p : 0.0;
       } else {
@@ -384,7 +398,7 @@ int ChunkF64::init(int n_, const double* l, const double* u, const double* w) {
     f.cls = tab.size();
     tab.resize(tab.size() + (T + 1) / 2, 0.0);
     std::memcpy(tab.data() + f.cls, cls.data(), sizeof(int) * T);
-    g_elems += (size_t)f.ncls * f.CP;
+    g_count += (size_t)f.ncls * f.C;
     cfgs.push_back(f);
   }
   if (cfgs.empty()) return NTK_OK;
@@ -396,24 +410,29 @@ int ChunkF64::init(int n_, const double* l, const double* u, const double* w) {
 }
 
 void ChunkF64::g_rows(const double* g, double* out) const {
+  SoftFactor* sg = reinterpret_cast<SoftFactor*>(out);
+  double* plain = out + 2 * g_count;
   for (const Cfg& f : cfgs)
     for (int j = 0; j < f.ncls; ++j)
-      for (int k = 0; k < f.CP; ++k) {
+      for (int k = 0; k < f.C; ++k) {
         const int r = f.rep[j] * f.C + k;
-        out[f.g + (size_t)j * f.CP + k] = k < f.C && r < n ? g[r] : 0.0;
+        const size_t at = f.g + (size_t)j * f.C + k;
+        plain[at] = r < n ? g[r] : 0.0;
+        sg[at] = soft_factor(plain[at]);
       }
 }
 
-// Costs in FP64 warp instructions of one sub-partition (~73 clocks each).
-// Chunks: a CTA's threads run C (5 + extra) row instructions, the two scans
-// and ~14 instructions' worth of staging and barriers; an SM's share of them
-// runs at the pipe's rate plus, once per wave of resident CTAs, the length of
-// one CTA's dependent chain.  One thread per system: n (3 + extra)
-// instructions a warp, times the measured distance from the pipe's rate, which
-// falls with the number of warps that hide each other's loads (a sub-partition
-// needs several; 512 rows, us, thread-per-system against chunks: contiguous
-// 4096 systems 179 : 29, 16384 181 : 104, 65536 362 : 363; strided compact
-// 16384 162 : 124, 49152 251 : 331).
+// Costs in FP64 warp instructions of one sub-partition (~76 clocks each).
+// Chunks: C (4 + extra) row instructions and the two scans for each CTA of an
+// SM's share, plus twice the length of one CTA's dependent chain (the first
+// CTAs fill the pipe and the last ones drain it; more where a second wave
+// starts late); row segments of strided systems below 128 bytes cost up to an
+// eighth.  One thread per system: n (3 + extra) instructions a warp times the
+// measured distance from the pipe's rate, which falls as more warps hide each
+// other's loads.  Measured, us, one thread a system against chunks: 512 rows
+// contiguous, 4096 systems 161 : 23, 16384 163 : 75, 65536 291 : 273, compact
+// with 262144 1169 : 1272; strided compact, 13472 systems of 333 rows 79 : 56,
+// 79990 240 : 275.
 const ChunkF64::Cfg* chunk_f64_pick(const ChunkF64& c, const Batch& b, int rhs, int* S) {
   const bool strided = b.es != 1;
   const int extra = rhs == RHS_COMPACT ? 1 : 0;
@@ -425,10 +444,11 @@ const ChunkF64::Cfg* chunk_f64_pick(const ChunkF64& c, const Batch& b, int rhs, 
       const size_t smem = smem_bytes(f, c.n, s, strided);
       const long long ctas = (b.nsys + s - 1) / s;
       if (nt < 32 || nt > 512 || smem > SMEM_MAX || ctas > 0x7fffffffLL) continue;
-      const double per_sm = std::ceil((double)ctas / SMS);
+      const double per_sm = std::max(1.0, (double)ctas / SMS + 0.5);
       const double resident = std::min<double>(std::min(32, 2048 / nt), SMEM_SM / (smem + 1024));
-      const double unit = f.C * (5 + extra) + 2 * log2_of(f.T) + 14;
-      const double cost = unit * (per_sm * nt / 128 + std::ceil(per_sm / resident));
+      const double work = f.C * (4 + extra) + 2 * log2_of(f.T) + 2;
+      const double cost = (work * per_sm * nt / 128 + (work + 12) * (per_sm > resident ? 2.5 : 2.0)) *
+                          (!strided || s == 16 ? 1.0 : s == 8 ? 1.05 : 1.12);
       if (!best || cost < best_cost) {
         best_cost = cost;
         best = &f;
@@ -436,24 +456,26 @@ const ChunkF64::Cfg* chunk_f64_pick(const ChunkF64& c, const Batch& b, int rhs, 
       }
     }
   const double load = std::ceil((double)((b.nsys + 31) / 32) / (4 * SMS));
-  const double far = strided ? 1.05 + 0.65 / load : 1.15 + 1.9 / load;
+  const double far = strided ? 0.97 + 0.55 / load : 0.95 + 1.5 / load;
   return best && best_cost < load * c.n * (3 + extra) * far ? best : nullptr;
 }
 
 int launch_chunk_f64(const ChunkF64& cf, const ChunkF64::Cfg& cfg, int S, const double* in, double* out,
-                     const Batch& b, const RhsParams& rp, const TablesF64& t, const double* g, cudaStream_t st) {
+                     const Batch& b, const RhsParams& rp, const TablesF64& t, cudaStream_t st) {
   const bool strided = b.es != 1;
   ChunkParams c;
   c.n = cf.n;
   c.S = S;
   c.T = cfg.T;
   c.C = cfg.C;
-  c.CP = cfg.CP;
-  c.P = pitch(cfg, cf.n);
+  c.P = pitch(cfg);
+  c.invC = 0xffffffffu / (unsigned)cfg.C + 1u;
   c.steps = log2_of(cfg.T);
   c.shift = strided ? log2_of(S) : c.steps;
   c.tab = cf.d_tab + cfg.tab;
-  c.g = g + cfg.g;
+  const double* rows = t.g + ChunkF64::g_offset(cf.n);
+  c.sg = reinterpret_cast<const SoftFactor*>(rows) + cfg.g;
+  c.g = rows + 2 * cf.g_count + cfg.g;
   c.scan = cf.d_tab + cfg.scan;
   c.cls = reinterpret_cast<const int*>(cf.d_tab + cfg.cls);
   c.plain = t;

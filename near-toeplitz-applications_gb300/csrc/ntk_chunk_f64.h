@@ -4,6 +4,7 @@
 #include <vector>
 
 #include "ntk_internal.h"
+#include "ntk_soft_f64.cuh"
 
 namespace ntk {
 
@@ -11,25 +12,28 @@ namespace ntk {
 struct ChunkF64 {
   struct Cfg {
     int T = 0;             // threads per system
-    int C = 0;             // rows per thread (odd: conflict-free in a dense shared-memory row)
-    int CP = 0;            // C rounded up to the row batch of the sweeps
+    int C = 0;             // rows per thread, a multiple of the sweeps' row batch
     int ncls = 0;          // distinct chunks (threads with bitwise equal factors share one)
-    size_t tab = 0;        // offset of [ncls][4][CP] -l, phi, -w, psi in d_tab
+    size_t tab = 0;        // offset of the classes' tables in d_tab
     size_t scan = 0;       // offset of [2][log2 T][T] scan multipliers in d_tab
     size_t cls = 0;        // offset of the T class numbers (ints) in d_tab
-    size_t g = 0;          // offset of [ncls][CP] rows of g among the g rows
+    size_t g = 0;          // offset of [ncls][C] rows of g among the g rows
     std::vector<int> rep;  // representative thread of each class
   };
   int n = 0;
   std::vector<Cfg> cfgs;
   double* d_tab = nullptr;
-  size_t g_elems = 0;      // values of the g rows of all configurations
+  size_t g_count = 0;      // rows of g of all configurations
 
   ~ChunkF64();
   // l, u: the matrix's LU factors, w = c / u.  Leaves cfgs empty where no
   // thread count applies; fails only where an allocation or a copy does.
   int init(int n, const double* l, const double* u, const double* w);
-  // rows of g[n] in chunk order for every configuration (g_elems values)
+  // A g table holds g[n] and, from g_offset(n) on, the rows of g in chunk
+  // order for every configuration, prepared for soft_product and plain
+  // (g_elems() doubles, filled by g_rows).
+  static size_t g_offset(int n) { return ((size_t)n + 1) & ~(size_t)1; }
+  size_t g_elems() const { return 3 * g_count; }
   void g_rows(const double* g, double* out) const;
 };
 
@@ -40,8 +44,8 @@ const ChunkF64::Cfg* chunk_f64_pick(const ChunkF64& c, const Batch& b, int rhs, 
 // rp.kind: RHS_IDENTITY, RHS_COMPACT or RHS_CROSS (with rp.center == 0 the
 // stencil is -(lo + hi): rows divided by -rp.top).  t: the matrix's plain
 // tables (systems whose values overflow or are not finite are solved with
-// them, row by row); g: the g rows of chunk order in device memory.
+// them, row by row), t.g a g table.
 int launch_chunk_f64(const ChunkF64& c, const ChunkF64::Cfg& cfg, int S, const double* in, double* out,
-                     const Batch& b, const RhsParams& rp, const TablesF64& t, const double* g, cudaStream_t st);
+                     const Batch& b, const RhsParams& rp, const TablesF64& t, cudaStream_t st);
 
 }  // namespace ntk

@@ -70,7 +70,7 @@ struct Plan {
   std::vector<double> lu_l, lu_u;   // host LU factors (FP64)
   double* d_lw = nullptr;           // device: l[n], w[n]
   ChunkF64 chunk;                   // NTK_FP64 with few systems: T threads per system
-  std::map<double, double*> g_by_scale;  // device g = s/u per RHS scale: g[n], then chunk's g rows
+  std::map<double, double*> g_by_scale;  // device g tables (g = s/u) per RHS scale
   RefineState* refine = nullptr;
   LongRefine* long_refine = nullptr;  // FP32 / FP32+refine windows for n > 1024
   SpikeSolver* spike = nullptr;       // n > 1024 where the windows' halos do not decay: exact partitions
