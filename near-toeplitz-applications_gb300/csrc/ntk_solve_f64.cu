@@ -16,7 +16,11 @@
 //   backward  x_i  = g_i * eta_i - w_i * x_{i+1}     (1 DMUL off the chain + 1 DFMA)
 // i.e. 3 (in-place solve) or 4 (fused compact derivative) FP64 instructions
 // per unknown, against ~10 plus two FP64 divisions per unknown in the
-// reference's cyclic reduction.  The forward values eta are parked in the
+// reference's cyclic reduction.  Nothing else may touch the FP64 pipe in the
+// row loops: a condition on the row (first, last) around FP64 work becomes
+// predicated instructions there, which hold the pipe like executed ones, so
+// the end rows are handled outside (512^3 derivatives: x 1446 -> 1169 us, y
+// 1157 -> 1030 us, 4 instructions a row alone 1033 us).  The forward values eta are parked in the
 // output array (they are L2-resident until the backward pass overwrites them
 // with x), so no shared memory is needed and occupancy is set by registers.
 // Threads of a warp take adjacent systems: for y/z sweeps of a 3D field these
@@ -26,6 +30,7 @@
 
 #include "ntk_device.cuh"
 #include "ntk_internal.h"
+#include "ntk_soft_f64.cuh"
 
 namespace ntk {
 namespace {
@@ -128,37 +133,36 @@ __device__ __forceinline__ double forward_compact(const double* src, double* dst
                                                   const double* __restrict__ l, double sigma0, double sigmaN) {
   FwdStream<VEC> st;
   st.init(src, es, n);
-  double fa = 0.0, fb = 0.0;  // f_{j-2}, f_{j-1}
-  double eta = 0.0;
+  double fa = st.ring[0], fb = st.ring[1];  // f_{j-2}, f_{j-1}
+  double eta = sigma0 * ((-5.0 * fa + 4.0 * fb) + (n > 2 ? st.ring[2] : 0.0));
   auto consume = [&](int j, double fc) {
-    if (j == 0) {
-      fb = fc;
-    } else if (j == 1) {
-      fa = fb;
-      fb = fc;
-    } else {
-      if (j == 2) {
-        eta = sigma0 * ((-5.0 * fa + 4.0 * fb) + fc);
-        dst[0] = eta;
-      }
-      eta = fma(-__ldg(l + (j - 1)), eta, fc - fa);
-      dst[(long long)(j - 1) * es] = eta;
-      fa = fb;
-      fb = fc;
-    }
+    eta = fma(-__ldg(l + (j - 1)), eta, fc - fa);
+    dst[(long long)(j - 1) * es] = eta;
+    fa = fb;
+    fb = fc;
   };
   int i0 = 0;
-  for (; i0 + PF <= n; i0 += PF) {
+  if (n >= PF) {  // the first block: rows 0 and 1 only enter the window
 #pragma unroll
     for (int k = 0; k < PF; ++k) {
-      const int i = i0 + k;
-      const double v = st.take(k, i);
-      consume(i, v);
+      const double v = st.take(k, k);
+      if (k == 1) dst[0] = eta;
+      if (k > 1) consume(k, v);
     }
+    for (i0 = PF; i0 + PF <= n; i0 += PF) {
+#pragma unroll
+      for (int k = 0; k < PF; ++k) {
+        const int i = i0 + k;
+        const double v = st.take(k, i);
+        consume(i, v);
+      }
+    }
+  } else {
+    dst[0] = eta;
   }
 #pragma unroll
   for (int k = 0; k < PF; ++k)
-    if (i0 + k < n) consume(i0 + k, st.ring[k]);
+    if (i0 + k > 1 && i0 + k < n) consume(i0 + k, st.ring[k]);
   return eta;  // eta_{n-2}; the caller closes row n-1
 }
 
@@ -458,7 +462,8 @@ __global__ void __launch_bounds__(32 * XWARPS) thomas_f64_xpose_kernel(const dou
   // ---- forward: eta_i, tiles of f in, tiles of eta out ----
   double eta = 0.0;
   double fm = 0.0, fc = 0.0;  // compact: f_{i-1}, f_i
-  double fl0 = 0.0, fl1 = 0.0, fl2 = 0.0;
+  double fl0 = 0.0;            // compact: f_{i-2}
+  double eta0 = 0.0;           // row 0, stored once row 1 has been read
   xtile_issue(ring, src, b.is, cnt, 0, n, lane);
   if (C > 1) xtile_issue(ring + XT * XP, src, b.is, cnt, XT, n, lane);
   for (int c = 0; c < C; ++c) {
@@ -480,38 +485,35 @@ __global__ void __launch_bounds__(32 * XWARPS) thomas_f64_xpose_kernel(const dou
       for (int k = 0; k < rows; ++k) {
         const int i = row0 + k;
         const double v = cur[k * XP + lane];
-        eta = (i == 0) ? v : fma(-__ldg(t.l + i), eta, v);
+        eta = fma(-__ldg(t.l + i), eta, v);  // l_0 = 0
         cur[k * XP + lane] = eta;
       }
     } else {
       if (c == 0) {
         fm = cur[0 * XP + lane];
         fc = cur[1 * XP + lane];
-        eta = rp.sigma0 * ((-5.0 * fm + 4.0 * fc) + cur[2 * XP + lane]);
+        eta = one_sided(rp.sigma0, fm, fc, cur[2 * XP + lane]);
+        eta0 = eta;
       }
+      // rows 1 .. n-2 of this tile; row n-1 closes the system below (a
+      // condition on the row inside the unrolled loop would become predicated
+      // FP64 instructions, which hold the pipe like executed ones)
+      const int last = min(rows, n - 1 - row0);
 #pragma unroll 8
-      for (int k = 0; k < rows; ++k) {
+      for (int k = c == 0 ? 1 : 0; k < last; ++k) {
         const int i = row0 + k;
-        if (i == 0) {
-          cur[lane] = eta;
-          continue;
-        }
-        if (i == n - 1) {
-          eta = fma(-__ldg(t.l + i), eta, rp.sigmaN * ((-5.0 * fl2 + 4.0 * fl1) + fl0));
-          cur[k * XP + lane] = eta;
-          continue;
-        }
         // f_{i+1}: next row of this tile or the first row of the next tile
         const double fp = (k + 1 < XT) ? cur[(k + 1) * XP + lane] : nxt[lane];
-        if (i == n - 3) fl0 = fc;
         eta = fma(-__ldg(t.l + i), eta, fp - fm);
+        fl0 = fm;
         fm = fc;
         fc = fp;
-        if (i == n - 2) {
-          fl1 = fm;
-          fl2 = fc;
-        }
         cur[k * XP + lane] = eta;
+      }
+      if (c == 0) cur[lane] = eta0;
+      if (row0 + rows == n) {  // fl0, fm, fc: f_{n-3}, f_{n-2}, f_{n-1}
+        eta = fma(-__ldg(t.l + (n - 1)), eta, one_sided(rp.sigmaN, fc, fm, fl0));
+        cur[(n - 1 - row0) * XP + lane] = eta;
       }
     }
     __syncwarp();
@@ -543,7 +545,7 @@ __global__ void __launch_bounds__(32 * XWARPS) thomas_f64_xpose_kernel(const dou
     for (int k = rows - 1; k >= 0; --k) {
       const int i = row0 + k;
       const double e = cur[k * XP + lane];
-      x = (i == n - 1) ? __ldg(t.g + i) * e : fma(-__ldg(t.w + i), x, __ldg(t.g + i) * e);
+      x = fma(-__ldg(t.w + i), x, __ldg(t.g + i) * e);
       cur[k * XP + lane] = x;
     }
     __syncwarp();
