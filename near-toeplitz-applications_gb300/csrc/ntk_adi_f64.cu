@@ -28,7 +28,10 @@
 // is 256 contiguous bytes.  (Folding 1/u into per-row stencil coefficients
 // saves one FP64 multiply per row but needs two more tables: measured
 // slower, and it moved the r = 40 error from below to above 1e-13.)
-// FP64 work per row: 3 (stencil; 1 when scaled) + 3 (sweeps) + 2 (carries).
+// FP64 work per row: 3 (stencil; 1 when scaled) + 2 (sweeps) + 2 (carries),
+// and 10 per lane for the scans (multipliers tabulated); the division by u
+// runs on the integer pipes (ntk_soft_f64.cuh).  A step of 2048 x 2048 (dt =
+// dx^2) 154 -> 131 us, of 999 x 999 52 -> 43.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -37,6 +40,7 @@
 #include "ntk_adi_geom.h"
 #include "ntk_plan.h"
 #include "ntk_refine.cuh"
+#include "ntk_soft_f64.cuh"
 
 namespace ntk {
 
@@ -45,7 +49,15 @@ namespace adi_f64_detail {
 using refine_detail::sys_pitch;
 using refine_detail::tile_off;
 
-constexpr int NTAB = 5;  // -l, phi, 1/u, -c/u, psi per row
+// Per window kind: [row in chunk][lane] tables of -l, phi, 1/u, -c/u, psi and
+// (16 bytes a row) 1/u prepared for soft_product, then the scans' multipliers
+// [2][5][lane].
+constexpr int NTAB = 5;
+constexpr int SCAN = 2 * 5 * 32;
+template <int M>
+__host__ __device__ constexpr int kind_pitch() {
+  return (NTAB + 2) * 32 * M + SCAN;
+}
 constexpr unsigned FULL = 0xffffffffu;
 
 template <int M>
@@ -54,7 +66,7 @@ __host__ __device__ constexpr size_t smem_bytes(int W) {
 }
 
 // One launch per half step: CTA b solves window b / nblk of the W
-// consecutive systems starting at (b % nblk) W.  tab: [kind][NTAB][M][32].
+// consecutive systems starting at (b % nblk) W.  tab: [kind][kind_pitch].
 template <int M, bool SCALED>
 __global__ void __launch_bounds__(256, 3)
     adi_f64_kernel(const double* __restrict__ in, double* __restrict__ out, AdiGeom geo,
@@ -95,12 +107,14 @@ __global__ void __launch_bounds__(256, 3)
   const int cb = lane * (M + 1);
   const long long s = s0 + warp;
   // row k of this lane's chunk in table t: tk[t * LW + 32 k]
-  const double* tk = tab + (size_t)wr.kind * NTAB * LW + lane;
+  const double* tk = tab + (size_t)wr.kind * kind_pitch<M>() + lane;
   const double* t_ml = tk;
   const double* t_phi = tk + LW;
   const double* t_iu = tk + 2 * LW;
   const double* t_mcu = tk + 3 * LW;
   const double* t_psi = tk + 4 * LW;
+  const uint4* t_siu = reinterpret_cast<const uint4*>(tk - lane + NTAB * LW) + lane;
+  const double* t_scan = tk + (NTAB + 2) * LW;  // step q: 32 q on, from the other end 32 (5 + q)
   double v[M];
   if (warp < wc) {
     const double* lo = lines + (size_t)warp * P + cb;
@@ -125,35 +139,43 @@ __global__ void __launch_bounds__(256, 3)
 #pragma unroll
   for (int k = 1; k < M; ++k) v[k] = fma(__ldg(t_ml + 32 * k), v[k - 1], v[k]);
   {
-    double a = v[M - 1], b = __ldg(t_phi + 32 * (M - 1));
+    double a = v[M - 1];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double ap = __shfl_up_sync(FULL, a, o);
-      const double bp = __shfl_up_sync(FULL, b, o);
-      if (lane >= o) {
-        a = fma(b, ap, a);
-        b *= bp;
-      }
+    for (int q = 0; q < 5; ++q) {
+      const double ap = __shfl_up_sync(FULL, a, 1 << q);
+      if (lane >= 1 << q) a = fma(__ldg(t_scan + 32 * q), ap, a);
     }
     double carry = __shfl_up_sync(FULL, a, 1);
     if (lane == 0) carry = 0.0;
 #pragma unroll
     for (int k = 0; k < M; ++k) v[k] = fma(__ldg(t_phi + 32 * k), carry, v[k]);
   }
-  // ---- backward ----
-  v[M - 1] *= __ldg(t_iu + 32 * (M - 1));
+  // ---- backward: y / u on the integer pipes, off the dependent chain ----
 #pragma unroll
-  for (int k = M - 2; k >= 0; --k) v[k] = fma(__ldg(t_mcu + 32 * k), v[k + 1], v[k] * __ldg(t_iu + 32 * k));
+  for (int k = M - 4; k >= 0; k -= 4) {
+    double y[4];
+    bool in_range = true;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const uint4 f4 = __ldg(t_siu + 32 * (k + q));
+      const SoftFactor f{(uint64_t)f4.y << 32 | f4.x, f4.z, f4.w};
+      in_range = in_range && soft_in_range(v[k + q], f);
+      y[q] = soft_product(v[k + q], f);
+    }
+    if (!in_range) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) y[q] = rare_mul(v[k + q], __ldg(t_iu + 32 * (k + q)));
+    }
+#pragma unroll
+    for (int q = 3; q >= 0; --q)
+      v[k + q] = k + q == M - 1 ? y[q] : fma(__ldg(t_mcu + 32 * (k + q)), v[(k + q + 1) % M], y[q]);
+  }
   {
-    double a = v[0], b = __ldg(t_psi);
+    double a = v[0];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const double ap = __shfl_down_sync(FULL, a, o);
-      const double bp = __shfl_down_sync(FULL, b, o);
-      if (lane + o < 32) {
-        a = fma(b, ap, a);
-        b *= bp;
-      }
+    for (int q = 0; q < 5; ++q) {
+      const double ap = __shfl_down_sync(FULL, a, 1 << q);
+      if (lane + (1 << q) < 32) a = fma(__ldg(t_scan + 32 * (5 + q)), ap, a);
     }
     double carry = __shfl_down_sync(FULL, a, 1);
     if (lane == 31) carry = 0.0;
@@ -200,7 +222,7 @@ struct AdiF64 {
   bool scaled = false;         // centre coefficient 0: rows divided by 1/dx^2
   double bottom = 0.0, center = 0.0, top = 0.0;
   int wx = 4, wy = 8;          // systems per CTA: x half step (rows), y half step (columns)
-  double* d_tab = nullptr;     // [4][NTAB][Lw]
+  double* d_tab = nullptr;     // [4][kind_pitch]
   ~AdiF64() {
     if (d_tab) cudaFree(d_tab);
   }
@@ -227,6 +249,22 @@ bool window_tables(int Lw, int M, const double co[7], double* t) {
   const std::vector<double>* tabs[5] = {&ml, &phi, &iu, &mcu, &psi};
   for (int q = 0; q < 5; ++q)
     for (int i = 0; i < Lw; ++i) t[(size_t)q * Lw + (i % M) * 32 + i / M] = (*tabs[q])[i];
+  SoftFactor* siu = reinterpret_cast<SoftFactor*>(t + (size_t)5 * Lw);
+  for (int i = 0; i < Lw; ++i) siu[(i % M) * 32 + i / M] = soft_factor(iu[i]);
+  // step q of a scan combines lane j with lane j -+ 2^q: the product of the
+  // chunks' responses between them, 0 beyond the first (last) lane
+  double* up = t + (size_t)7 * Lw;
+  double* down = up + 5 * 32;
+  for (int j = 0; j < 32; ++j) {
+    up[j] = j > 0 ? phi[j * M + M - 1] : 0.0;
+    down[j] = j < 31 ? psi[j * M] : 0.0;
+  }
+  for (int q = 1; q < 5; ++q)
+    for (int j = 0; j < 32; ++j) {
+      const int o = 1 << (q - 1);
+      up[32 * q + j] = j >= 2 * o ? up[32 * (q - 1) + j] * up[32 * (q - 1) + j - o] : 0.0;
+      down[32 * q + j] = j + 2 * o < 32 ? down[32 * (q - 1) + j] * down[32 * (q - 1) + j + o] : 0.0;
+    }
   return true;
 }
 
@@ -329,7 +367,7 @@ int adi_f64_create(AdiF64** out, int N, double dx, double dt) {
   const double last[7] = {bi, ei, ei, bi, ei, 0.0, 1.0};
   const double wholem[7] = {1.0, 0.0, ei, bi, ei, 0.0, 1.0};
   const double* co[4] = {first, middle, last, wholem};
-  const size_t per = (size_t)adi_f64_detail::NTAB * Lw;
+  const size_t per = (size_t)(adi_f64_detail::NTAB + 2) * Lw + adi_f64_detail::SCAN;
   std::vector<double> host(4 * per, 0.0);
   for (int k = 0; k < 4; ++k) {
     if ((k == 3) != whole) continue;
