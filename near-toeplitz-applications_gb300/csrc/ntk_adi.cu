@@ -15,8 +15,9 @@
 // In FP64 each half step solves overlapping windows of 32 M rows, one warp
 // per window (ntk_adi_f64.cu), when N >= 128 and the factors decay fast
 // enough for a halo exact to rounding (r = 0.5: |l| -> 0.268, 36 rows);
-// otherwise the segmented FP64 sweeps (ntk_solve_f64.cu) with the largest
-// exact segmentation.
+// otherwise whole systems, several threads each (ntk_chunk_f64.cu, nothing
+// truncated), and where a system is too long for that the segmented FP64
+// sweeps (ntk_solve_f64.cu) with the largest exact segmentation.
 // In FP32 + refinement the half steps solve overlapping windows as well
 // (ntk_adi_refine.cu); where their factors decay too slowly for an exact
 // halo (large r), a step runs the reference's six kernels instead, with the
@@ -47,7 +48,12 @@ struct Adi {
   SegParams sp;
   double bottom = 0, center = 0, top = 0;
   AdiRefine* refine = nullptr;  // NTK_FP32 / NTK_FP32_REFINE half steps (ntk_adi_refine.cu)
-  AdiF64* windows = nullptr;    // NTK_FP64 window half steps (ntk_adi_f64.cu), else segmented sweeps
+  // NTK_FP64: window half steps (ntk_adi_f64.cu), else whole systems in shared
+  // memory (ntk_chunk_f64.cu; `rows` holds their matrix, divided by 1/dx^2
+  // where the stencil's centre is zero), else segmented sweeps
+  AdiF64* windows = nullptr;
+  Plan rows;
+  bool chunks = false;
   SpikeSolver* spike = nullptr;  // FP32 / FP32 + refinement rows where the windows do not apply
   cudaStream_t capture_stream = nullptr;
   std::map<std::tuple<const void*, const void*, const void*, int>, cudaGraphExec_t> graphs;
@@ -110,7 +116,47 @@ int adi_spike_step(Adi* a, double* u, double* d_x, const double* d_y, cudaStream
 
 }  // namespace
 
+namespace {
+
+// The x half step's systems (rows 1 .. N-2 from u + N to d_x + N) and the y
+// half step's (columns 1 .. N-2 from d_x + 1 to u + 1), with their stencils
+// and boundary values.
+void half_systems(const Adi* a, const double* d_x, const double* d_y, Batch* bx, RhsParams* rx, Batch* by,
+                  RhsParams* ry) {
+  const int N = a->N;
+  bx->nsys = bx->ni = N - 2;
+  bx->is = N;
+  bx->es = 1;
+  rx->kind = RHS_CROSS;
+  rx->bottom = a->bottom;
+  rx->center = a->center;
+  rx->top = a->top;
+  rx->cs = N;
+  rx->bnd = d_x + N;
+  rx->bnd_ss = N;
+  rx->bnd_es = 1;
+  *by = *bx;
+  by->is = 1;
+  by->es = N;
+  *ry = *rx;
+  ry->cs = 1;
+  ry->bnd = d_y + N;
+}
+
+// Both half steps over whole systems (ntk_chunk_f64.cu).
+int adi_chunk_step(Adi* a, double* u, double* d_x, const double* d_y, cudaStream_t st) {
+  Batch bx, by;
+  RhsParams rx, ry;
+  half_systems(a, d_x, d_y, &bx, &rx, &by, &ry);
+  int rc = a->rows.run_chunks(u + a->N, d_x + a->N, bx, rx, 1.0, st);
+  if (!rc) rc = a->rows.run_chunks(d_x + 1, u + 1, by, ry, 1.0, st);
+  return rc;
+}
+
+}  // namespace
+
 int adi_step(Adi* a, double* u, double* d_x, const double* d_y, cudaStream_t st) {
+  if (a->chunks) return adi_chunk_step(a, u, d_x, d_y, st);
   if (a->spike) return adi_spike_step(a, u, d_x, d_y, st);
   if (a->refine) return adi_refine_step(a->refine, u, d_x, d_y, st);
   if (a->windows) return adi_f64_step(a->windows, u, d_x, d_y, st);
@@ -120,36 +166,11 @@ int adi_step(Adi* a, double* u, double* d_x, const double* d_y, cudaStream_t st)
   t.w = a->plan.d_lw + N;
   int rc = a->plan.g_table(1.0, &t.g);
   if (rc) return rc;
-  // x half step
-  Batch bx;
-  bx.nsys = N - 2;
-  bx.ni = N - 2;
-  bx.is = N;
-  bx.os = 0;
-  bx.es = 1;
-  RhsParams rx;
-  rx.kind = RHS_CROSS;
-  rx.bottom = a->bottom;
-  rx.center = a->center;
-  rx.top = a->top;
-  rx.cs = N;
-  rx.bnd = d_x + N;
-  rx.bnd_ss = N;
-  rx.bnd_es = 1;
+  Batch bx, by;
+  RhsParams rx, ry;
+  half_systems(a, d_x, d_y, &bx, &rx, &by, &ry);
   rc = launch_thomas_f64_segmented(u + N, a->scratch + N, d_x + N, N, bx, rx, t, a->sp, st);
   if (rc) return rc;
-  // y half step
-  Batch by;
-  by.nsys = N - 2;
-  by.ni = N - 2;
-  by.is = 1;
-  by.os = 0;
-  by.es = N;
-  RhsParams ry = rx;
-  ry.cs = 1;
-  ry.bnd = d_y + N;
-  ry.bnd_ss = N;
-  ry.bnd_es = 1;
   return launch_thomas_f64_segmented(d_x + 1, a->scratch + 1, u + 1, N, by, ry, t, a->sp, st);
 }
 
@@ -193,10 +214,21 @@ int ntk_adi_create(ntk_adi** out, int N, double dx, double dt, int precision) {
     for (int i = 0; i < N; ++i) w[i] = (i < N - 1 ? a->plan.mat.c(i) : 0.0) / a->plan.lu_u[i];
     a->sp = ntk::choose_segments(a->plan.lu_l.data(), w.data(), N, N - 2);
     if (precision == NTK_FP64) {
-      // windows where they apply (N >= 128, fast enough decay), else the
-      // segmented sweeps with their N x N scratch array
+      // Windows where they apply (N >= 128, fast enough decay); else whole
+      // systems, several threads each, where one fits in shared memory
+      // (N = 64: 17 us a step against 81 of the segmented sweeps); else the
+      // segmented sweeps with their N x N scratch array.
       rc = ntk::adi_f64_create(&a->windows, N, dx, dt);
-      if (rc == NTK_ERR_UNSUPPORTED)
+      if (rc == NTK_ERR_UNSUPPORTED) rc = NTK_OK;
+      if (rc == NTK_OK && !a->windows) {
+        const double e = a->center == 0.0 ? 1. / (dx * dx) : 1.0;
+        const double rows[7] = {1., 0., co[2] / e, co[3] / e, co[4] / e, 0., 1.};
+        rc = a->rows.init(N, N - 2, rows, NTK_FP64, 1);
+        a->chunks = rc == NTK_OK && a->rows.chunk.serves_both_layouts();
+        const double* g = nullptr;  // made here, not by the first step, which may be under capture
+        if (a->chunks) rc = a->rows.g_table(1.0, &g);
+      }
+      if (rc == NTK_OK && !a->windows && !a->chunks)
         rc = ntk::cuda_status(cudaMalloc(&a->scratch, sizeof(double) * (size_t)N * N), "cudaMalloc(ADI scratch)");
     } else {
       rc = ntk::adi_refine_create(&a->refine, N, dx, dt, precision);
@@ -238,6 +270,13 @@ int ntk_adi_segments(const ntk_adi* adi, int* seg_len, int* halo, int* nseg) {
   if (!adi) {
     ntk::set_error("ntk_adi_segments: null plan");
     return NTK_ERR_INVALID;
+  }
+  if (adi->chunks) {
+    // whole systems
+    if (seg_len) *seg_len = adi->N;
+    if (halo) *halo = 0;
+    if (nseg) *nseg = 1;
+    return NTK_OK;
   }
   if (adi->spike) {
     // partitions of 512 rows, no halo

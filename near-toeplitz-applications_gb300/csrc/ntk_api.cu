@@ -168,6 +168,23 @@ int Plan::run(const double* in, double* out, const Batch& b, RhsParams rp, doubl
   return run_refine(in, out, b, rp, s, stream);
 }
 
+int Plan::run_chunks(const double* in, double* out, const Batch& b, const RhsParams& rp, double s,
+                     cudaStream_t stream) {
+  int rc = check_device();
+  if (rc || b.nsys == 0) return rc;
+  TablesF64 t;
+  t.l = d_lw;
+  t.w = d_lw + n;
+  if ((rc = g_table(s, &t.g))) return rc;
+  int S = 0;
+  const ChunkF64::Cfg* cfg = chunk_f64_pick(chunk, b, rp.kind, &S, true);
+  if (!cfg) {
+    set_error("no thread count serves this batch of systems of %d rows", n);
+    return NTK_ERR_UNSUPPORTED;
+  }
+  return launch_chunk_f64(chunk, *cfg, S, in, out, b, rp, t, stream);
+}
+
 static bool bad_ptr(const void* p) { return p == nullptr || (reinterpret_cast<uintptr_t>(p) & 7) != 0; }
 
 }  // namespace ntk

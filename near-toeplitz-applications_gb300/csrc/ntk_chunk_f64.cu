@@ -409,6 +409,12 @@ int ChunkF64::init(int n_, const double* l, const double* u, const double* w) {
   return rc;
 }
 
+bool ChunkF64::serves_both_layouts() const {
+  for (const Cfg& f : cfgs)  // contiguous systems fit every configuration kept by init
+    if (4 * f.T >= 32 && smem_bytes(f, n, 4, true) <= SMEM_MAX) return true;
+  return false;
+}
+
 void ChunkF64::g_rows(const double* g, double* out) const {
   SoftFactor* sg = reinterpret_cast<SoftFactor*>(out);
   double* plain = out + 2 * g_count;
@@ -433,7 +439,7 @@ void ChunkF64::g_rows(const double* g, double* out) const {
 // contiguous, 4096 systems 161 : 23, 16384 163 : 75, 65536 291 : 273, compact
 // with 262144 1169 : 1272; strided compact, 13472 systems of 333 rows 79 : 56,
 // 79990 240 : 275.
-const ChunkF64::Cfg* chunk_f64_pick(const ChunkF64& c, const Batch& b, int rhs, int* S) {
+const ChunkF64::Cfg* chunk_f64_pick(const ChunkF64& c, const Batch& b, int rhs, int* S, bool always) {
   const bool strided = b.es != 1;
   const int extra = rhs == RHS_COMPACT ? 1 : 0;
   const ChunkF64::Cfg* best = nullptr;
@@ -455,6 +461,7 @@ const ChunkF64::Cfg* chunk_f64_pick(const ChunkF64& c, const Batch& b, int rhs, 
         *S = s;
       }
     }
+  if (always) return best;
   const double load = std::ceil((double)((b.nsys + 31) / 32) / (4 * SMS));
   const double far = strided ? 0.97 + 0.55 / load : 0.95 + 1.5 / load;
   return best && best_cost < load * c.n * (3 + extra) * far ? best : nullptr;

@@ -29,6 +29,8 @@ struct ChunkF64 {
   // l, u: the matrix's LU factors, w = c / u.  Leaves cfgs empty where no
   // thread count applies; fails only where an allocation or a copy does.
   int init(int n, const double* l, const double* u, const double* w);
+  // whether some configuration fits contiguous and some strided systems
+  bool serves_both_layouts() const;
   // A g table holds g[n] and, from g_offset(n) on, the rows of g in chunk
   // order for every configuration, prepared for soft_product and plain
   // (g_elems() doubles, filled by g_rows).
@@ -38,8 +40,9 @@ struct ChunkF64 {
 };
 
 // The configuration for a batch, or null where one thread per system
-// (ntk_solve_f64.cu) is the faster; S: systems per CTA.
-const ChunkF64::Cfg* chunk_f64_pick(const ChunkF64& c, const Batch& b, int rhs, int* S);
+// (ntk_solve_f64.cu) is the faster and `always` is not set, or where none
+// fits; S: systems per CTA.
+const ChunkF64::Cfg* chunk_f64_pick(const ChunkF64& c, const Batch& b, int rhs, int* S, bool always = false);
 
 // rp.kind: RHS_IDENTITY, RHS_COMPACT or RHS_CROSS (with rp.center == 0 the
 // stencil is -(lo + hi): rows divided by -rp.top).  t: the matrix's plain

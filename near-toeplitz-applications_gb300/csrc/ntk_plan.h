@@ -93,6 +93,10 @@ struct Plan {
   int check_device() const;
   int run(const double* in, double* out, const Batch& b, RhsParams rp, double s, cudaStream_t stream);
 
+  // several threads per system whatever the batch (NTK_FP64 plans whose chunk
+  // tables serve the layout)
+  int run_chunks(const double* in, double* out, const Batch& b, const RhsParams& rp, double s, cudaStream_t stream);
+
   // FP32 / FP32 + refinement (ntk_refine.cu)
   int init_refine();
   int run_refine(const double* in, double* out, const Batch& b, const RhsParams& rp, double s, cudaStream_t stream);
