@@ -59,7 +59,8 @@ int ntk_last_error(char* buf, int len);
  * windows (NTK_ERR_UNSUPPORTED when the LU multipliers |a/u|, |c/u| of the
  * interior are >= 0.9, too slow a decay for the windows), and an in-place
  * call on them copies its input to a work array the plan allocates on first
- * use.  Synchronous. */
+ * use (not where all windows of a system are solved by one CTA).
+ * Synchronous. */
 int ntk_plan_create(ntk_plan** out, int n, long long nrhs, const double coeffs[7], int precision,
                     int refine_sweeps);
 
@@ -87,7 +88,11 @@ int ntk_plan_create(ntk_plan** out, int n, long long nrhs, const double coeffs[7
  *                           groups solved while a third loads (3); 0
  *                           (default) picks 3 for NTK_FP32 and 2 for
  *                           NTK_FP32_REFINE (faster on GB300); 1 the
- *                           chunked kernel above.  With 0, 2 or 3,
+ *                           chunked kernel above.  Other n >= 64 and
+ *                           layouts, one sweep: 1 the chunked kernel, else
+ *                           paired chunks of any number where the factors
+ *                           decay within 16 rows and the batch fills the
+ *                           GPU.  With 0, 2 or 3,
  *                           NTK_TUNE_REFINE_W sets the systems per CTA of
  *                           contiguous layouts (4, 8 or 16).
  *   NTK_TUNE_REFINE_PREFETCH  the one-group strided kernel: a CTA prefetches

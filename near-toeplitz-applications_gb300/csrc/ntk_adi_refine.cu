@@ -306,6 +306,7 @@ int adi_refine_create(AdiRefine** out, int N, double dx, double dt, int precisio
   const double* co[4] = {first, middle, last, whole};
   for (int k = 0; k < 4; ++k) {
     if ((k == 3) != ar->whole) continue;
+    ar->win[k].window_tables = true;
     int rc = ar->win[k].init(ar->Lw, 1, co[k], NTK_FP32_REFINE, 1);
     if (rc == NTK_OK) rc = ar->win[k].init_refine();
     if (rc) {

@@ -286,6 +286,7 @@ int long_refine_create(LongRefine** out, const Plan& p, int precision, int sweep
   const double last[7] = {co[3], co[4], co[2], co[3], co[4], co[5], co[6]};
   const double* kc[3] = {first, middle, last};
   for (int k = 0; k < 3; ++k) {
+    lr->win[k].window_tables = true;
     int rc = lr->win[k].init(LLW, 1, kc[k], NTK_FP32_REFINE, 1);
     if (rc == NTK_OK) rc = lr->win[k].init_refine();
     if (rc) {

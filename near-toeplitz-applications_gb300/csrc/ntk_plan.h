@@ -58,6 +58,7 @@ bool factor_host(const Matrix& m, std::vector<double>& l, std::vector<double>& u
 struct RefineState;  // ntk_refine.cu
 struct LongRefine;   // ntk_long_refine.cu
 struct SpikeSolver;  // ntk_spike.cu
+struct R2N;          // ntk_r2n.cu
 
 struct Plan {
   int n = 0;
@@ -74,6 +75,8 @@ struct Plan {
   RefineState* refine = nullptr;
   LongRefine* long_refine = nullptr;  // FP32 / FP32+refine windows for n > 1024
   SpikeSolver* spike = nullptr;       // n > 1024 where the windows' halos do not decay: exact partitions
+  bool window_tables = false;         // a window matrix of another plan: tables only, no batches of its own
+  R2N* r2n = nullptr;                 // one sweep, any n: paired chunks (null where they do not apply)
   LongRefine* long_alt = nullptr;     // 512 < n <= 1024: two-window solve (64 threads per system)
   std::mutex mu;
   // launch configuration (ntk_plan_set_tuning; chosen by the autotuner)

@@ -8,6 +8,7 @@
 #include "ntk_long_refine.h"
 #include "ntk_spike.h"
 #include "ntk_r2.h"
+#include "ntk_r2n.h"
 #include "ntk_refine.cuh"
 
 namespace ntk {
@@ -52,6 +53,10 @@ int Plan::init_refine() {
     return NTK_ERR_ALLOC;
   }
   refine = st;
+  if (precision == NTK_FP32_REFINE && sweeps == 1 && !window_tables) {
+    const int rc = r2n_create(&r2n, *this);
+    if (rc) return rc;
+  }
   int M = 0;
   for (int m : {4, 8, 16, 32})
     if (n <= 32 * m) {
@@ -193,6 +198,7 @@ void Plan::status_words(std::vector<unsigned*>& out) const {
   if (long_refine) long_refine_status_words(long_refine, out);
   if (spike) spike_status_words(spike, out);
   if (long_alt) long_refine_status_words(long_alt, out);
+  r2n_status_words(r2n, out);
 }
 
 void Plan::release_refine() {
@@ -208,6 +214,10 @@ void Plan::release_refine() {
     long_refine_destroy(long_alt);
     long_alt = nullptr;
   }
+  if (r2n) {
+    r2n_destroy(r2n);
+    r2n = nullptr;
+  }
   if (!refine) return;
   if (refine->d_tab) cudaFree(refine->d_tab);
   if (refine->d_status) cudaFree(refine->d_status);
@@ -217,6 +227,10 @@ void Plan::release_refine() {
 
 int Plan::run_refine(const double* in, double* out, const Batch& b, const RhsParams& rp, double s,
                      cudaStream_t stream) {
+  // every length but the 512-row kernels' own
+  const bool own_512 = refine && refine->r2_ok && r2::layout_ok(in, out, b);
+  if (!own_512 && tune_refine_kernel != 1 && tune_refine_tps != 64 && r2n_serves(r2n, in, out, b, rp))
+    return r2n_run(r2n, in, out, b, rp, s, tune_refine_prefetch, stream);
   if (spike) {
     if (rp.kind != RHS_IDENTITY || s != 1.0) {
       set_error("FP32/refine with slowly decaying LU factors (n > 1024) supports the plain solve only");
