@@ -316,8 +316,8 @@ template <int RHS, bool STRIDED>
 int launch_one(const double* in, double* out, const Batch& b, const RhsParams& rp, const ChunkParams& c, size_t smem,
                cudaStream_t st) {
   auto k = chunk_f64_kernel<RHS, STRIDED>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(chunk_f64_kernel)");
+  int rc = allow_smem(k, smem, "cudaFuncSetAttribute(chunk_f64_kernel)");
+  if (rc) return rc;
   const long long blocks = (b.nsys + c.S - 1) / c.S;
   k<<<(unsigned)blocks, c.S * c.T, smem, st>>>(in, out, b, rp, c);
   return cuda_status(cudaGetLastError(), "chunk_f64_kernel");

@@ -113,6 +113,14 @@ struct TablesF64 {
 void set_error(const char* fmt, ...);
 int cuda_status(cudaError_t e, const char* where);
 
+// Lets a kernel launch with smem bytes of dynamic shared memory; 48 KB need no
+// call (a call is ~1 us of a small launch's host time).
+template <class K>
+int allow_smem(K kernel, size_t smem, const char* where) {
+  if (smem <= 48 * 1024) return NTK_OK;
+  return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), where);
+}
+
 // Status bits the FP32 / FP32+refinement kernels raise in their device
 // status words (ntk.h NTK_STATUS_*).
 constexpr unsigned STATUS_RANGE = 1u;  // an input outside the double-word range (|x| >= 2^128, inf, nan)

@@ -719,8 +719,8 @@ int r2n_launch(const R2N* r, const CUtensorMap& map, const double* in, double* o
                const r2::Args& a, long long groups, cudaStream_t st) {
   auto k = r2n::r2n_kernel<RHS, CONTIG, GEN, SEQ>;
   const size_t smem = r2n::smem_of<CONTIG>(g.Wr, g.nc, SEQ ? g.H : 0);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(r2n_kernel)");
+  int rc = allow_smem(k, smem, "cudaFuncSetAttribute(r2n_kernel)");
+  if (rc) return rc;
   const long long grid = SEQ ? groups : groups * g.P;
   k<<<(unsigned)grid, r2n::SG * g.nc, smem, st>>>(map, in, out, g, a, r->d_tables);
   return cuda_status(cudaGetLastError(), "r2n_kernel");

@@ -668,8 +668,8 @@ int launch_one(const double* in, double* out, int n, const Batch& b, const Refin
   const int S = SPW * W;
   const size_t smem = refine_smem<M>(S, ra.ncls, b.es);
   auto kern = refine_kernel<M, RHS, SWEEPS, POW2, PAD, DECAY, SPW>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(refine_kernel)");
+  int rc = allow_smem(kern, smem, "cudaFuncSetAttribute(refine_kernel)");
+  if (rc) return rc;
   const long long blocks = (b.nsys + S - 1) / S;
   if (blocks > 0x7fffffffLL) {
     set_error("too many systems for one launch");
