@@ -53,7 +53,8 @@ using namespace r2;
 
 constexpr int SG = 16;        // systems per CTA
 constexpr int MAX_NC = 32;    // chunks of a window
-// exchange arrays, [chunk][system] floats each
+// exchange values, [chunk][value][system] floats: a neighbour's are a constant
+// distance away, and the two chunks of a warp use all 32 banks
 enum { X_E1 = 0, X_S1, X_A0, X_B0, X_B7, X_E2, X_S2, X_COUNT };
 
 // Factors of one chunk as pairs (row k, row k + 8).
@@ -186,7 +187,8 @@ __global__ void __launch_bounds__(512, 2)
   const int x0 = (grp - plane * g.gpp) * SG;
   const int live = min(SG, g.ni - x0);  // systems of this group
   const long long base = (long long)plane * g.os + (long long)x0 * g.is;
-  auto X = [&](int which, int chunk) -> float& { return xch[(which * g.nc + chunk) * SG + s]; };
+  float* xc = xch + c * (X_COUNT * SG) + s;
+  auto X = [&](int which, int d) -> float& { return xc[(d * X_COUNT + which) * SG]; };  // chunk c + d
   double* col = tile + (CONTIG ? s * (g.Wr + 2) : s);
   const long long mine = base + (long long)s * g.is;  // this system's row 0
   if (t == 0) mbar_init(bar, 1);
@@ -322,10 +324,6 @@ __global__ void __launch_bounds__(512, 2)
           h = bh;
           l = bl;
         }
-        if (tail && k >= kt) {
-          h = k == kt ? bh : 0.f;
-          l = k == kt ? bl : 0.f;
-        }
         if (k == 0) edge0 = make_float2(h, l);
         else if (k == ROWS - 1) edge15 = make_float2(h, l);
         else if (!CONTIG || k == 1 || k == ROWS - 2) put(k, h, l);
@@ -336,6 +334,18 @@ __global__ void __launch_bounds__(512, 2)
         else v[k - HALF].y = h;
         prev = cur;
         cur = nxt;
+      }
+      if (tail) {  // the last row's stencil, zeros beyond it
+#pragma unroll
+        for (int k = 0; k < ROWS; ++k)
+          if (k >= kt) {
+            const float h = k == kt ? bh : 0.f, l = k == kt ? bl : 0.f;
+            if (k == 0) edge0 = make_float2(h, l);
+            else if (k == ROWS - 1) edge15 = make_float2(h, l);
+            else put(k, h, l);
+            if (k < HALF) v[k % HALF].x = h;
+            else v[k % HALF].y = h;
+          }
       }
     } else {
       const bool keep = SEQ && w < g.P - 1 && r0 + ROWS > hi - g.H && r0 < hi;
@@ -378,7 +388,7 @@ __global__ void __launch_bounds__(512, 2)
 #pragma unroll
       for (int k = 0; k < HALF; ++k) v[k] = make_float2(0.f, 0.f);
     }
-    X(X_E1, c) = tab ? forward(v, ft) : forward(v, fc);
+    X(X_E1, 0) = tab ? forward(v, ft) : forward(v, fc);
     __syncthreads();  // carries published; every halo row has been read
     if (RHS == RHS_COMPACT) {
       put(0, edge0.x, edge0.y);
@@ -386,24 +396,24 @@ __global__ void __launch_bounds__(512, 2)
     }
     const bool from_left = c > 0 && !dead;
     {
-      const float CA = from_left ? X(X_E1, c - 1) : 0.f;
-      X(X_S1, c) = tab ? backward(v, CA, ft) : backward(v, CA, fc);
+      const float CA = from_left ? X(X_E1, -1) : 0.f;
+      X(X_S1, 0) = tab ? backward(v, CA, ft) : backward(v, CA, fc);
     }
-    X(X_A0, c) = v[0].x;
-    X(X_B0, c) = v[0].y;
-    X(X_B7, c) = v[7].y;
+    X(X_A0, 0) = v[0].x;
+    X(X_B0, 0) = v[0].y;
+    X(X_B7, 0) = v[7].y;
     __syncthreads();
     {
-      const float XB = c < last ? X(X_S1, c + 1) : 0.f;
+      const float XB = c < last ? X(X_S1, 1) : 0.f;
       if (tab) carry_in(v, XB, ft);
       else carry_in(v, XB, fc);
     }
     // ---- residual: the neighbours' edge rows as their owners have them ----
     float xl = 0.f, xr = 0.f;
-    if (from_left) xl = fma_(c == 1 ? tabs[0].psi[7].y : K.psi[7].y, X(X_S1, c), X(X_B7, c - 1));
+    if (from_left) xl = fma_(c == 1 ? tabs[0].psi[7].y : K.psi[7].y, X(X_S1, 0), X(X_B7, -1));
     if (c < last) {
-      const float XA = c + 1 < last ? fma_(K.psi[0].y, X(X_S1, c + 2), X(X_B0, c + 1)) : X(X_B0, c + 1);
-      xr = fma_(c + 1 == last ? tabs[1].psi[0].x : K.psi[0].x, XA, X(X_A0, c + 1));
+      const float XA = c + 1 < last ? fma_(K.psi[0].y, X(X_S1, 2), X(X_B0, 1)) : X(X_B0, 1);
+      xr = fma_(c + 1 == last ? tabs[1].psi[0].x : K.psi[0].x, XA, X(X_A0, 1));
     }
     float2 r[8];
     auto residual = [&](int k, float2 da, float2 db) {
@@ -453,15 +463,15 @@ __global__ void __launch_bounds__(512, 2)
       for (int k = 0; k < HALF; ++k) r[k] = make_float2(0.f, 0.f);
     }
     // ---- FP32 correction solve ----
-    X(X_E2, c) = tab ? forward(r, ft) : forward(r, fc);
+    X(X_E2, 0) = tab ? forward(r, ft) : forward(r, fc);
     __syncthreads();
     {
-      const float CA = from_left ? X(X_E2, c - 1) : 0.f;
-      X(X_S2, c) = tab ? backward(r, CA, ft) : backward(r, CA, fc);
+      const float CA = from_left ? X(X_E2, -1) : 0.f;
+      X(X_S2, 0) = tab ? backward(r, CA, ft) : backward(r, CA, fc);
     }
     __syncthreads();
     {
-      const float XB = c < last ? X(X_S2, c + 1) : 0.f;
+      const float XB = c < last ? X(X_S2, 1) : 0.f;
       if (tab) carry_in(r, XB, ft);
       else carry_in(r, XB, fc);
     }
@@ -493,13 +503,15 @@ __global__ void __launch_bounds__(512, 2)
       }
     } else {
       double* dst = out + mine + (long long)(start + r0) * g.es;
-      const int k0 = s < live ? lo - r0 : ROWS, k1 = hi - r0;  // rows of this chunk to store: k0 <= k < k1
+      // rows of this chunk to store: bits lo - r0 .. hi - r0 - 1
+      const unsigned below = (1u << min(max(lo - r0, 0), ROWS)) - 1u;
+      const unsigned rows = s < live ? ((1u << min(max(hi - r0, 0), ROWS)) - 1u) & ~below : 0u;
 #pragma unroll
       for (int k = 0; k < HALF; ++k) {
         double oa, ob;
         out_pair(v[k], r[k], a, oa, ob);
-        if (k >= k0 && k < k1) dst[(long long)k * g.es] = oa;
-        if (k + HALF >= k0 && k + HALF < k1) dst[(long long)(k + HALF) * g.es] = ob;
+        if (rows >> k & 1u) dst[(long long)k * g.es] = oa;
+        if (rows >> (k + HALF) & 1u) dst[(long long)(k + HALF) * g.es] = ob;
       }
     }
     if (!SEQ || ++w == g.P) break;
