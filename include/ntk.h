@@ -88,7 +88,7 @@ int ntk_plan_create(ntk_plan** out, int n, long long nrhs, const double coeffs[7
  *                           groups solved while a third loads (3); 0
  *                           (default) picks 3 for NTK_FP32 and 2 for
  *                           NTK_FP32_REFINE (faster on GB300); 1 the
- *                           chunked kernel above.  Other n >= 64 and
+ *                           chunked kernel above.  Other n >= 96 and
  *                           layouts, one sweep: 1 the chunked kernel, else
  *                           paired chunks of any number where the factors
  *                           decay within 16 rows and the batch fills the

@@ -6,8 +6,8 @@
 // every other length (ntk_refine.cuh) gives a system one warp of 4, 8, 16 or
 // 32 rows a lane: 385 rows pay for 512, 700 for 1024 (with a register file's
 // worth of rows per lane), 240 for 256 in 8-row chunks whose carries need
-// scans, at 110-124 instructions a row.  Here a CTA takes 16 systems and one
-// thread per system and 16-row chunk, nc = ceil(n / 16) chunks: nothing is
+// scans, at 110-124 instructions a row.  Here a CTA takes 16 systems (8
+// contiguous ones) and one thread per system and 16-row chunk, nc = ceil(n / 16) chunks: nothing is
 // paid for beyond the last chunk.  Systems longer than 512 rows are cut into
 // P equal windows of Wr rows overlapping by H-row halos (as in
 // ntk_long_refine.cu: the product of the multipliers over H rows is below
@@ -32,10 +32,10 @@
 //    (ntk_long_refine.cu copies the whole input first: 82 of 281 us for 16384
 //    systems of 2048 rows).
 // Measured against the chunked kernels, us: derivatives of a 240 x 385 x 700
-// field along x (700 rows) 814 -> 379, y (385) 448 -> 361, z (240) 439 -> 291;
-// 16384 systems of 2048 rows in place 282 -> 199, 65536 of 100 rows 60 -> 37,
-// 2600 of 300 rows 12.3 -> 11.5.  Below one 16-system group per SM the chunked
-// kernels keep the batch (eight systems a CTA spread it over more SMs).
+// field along x (700 rows) 814 -> 304, y (385) 448 -> 341, z (240) 439 -> 277;
+// 16384 systems of 2048 rows in place 281 -> 185, 65536 of 100 rows 60 -> 37,
+// 2600 of 300 rows 12.6 -> 10.5.  Below one group per SM the chunked kernels
+// keep the batch.
 #include "ntk_r2n.h"
 
 #include <algorithm>
@@ -51,10 +51,13 @@ namespace r2n {
 
 using namespace r2;
 
-constexpr int SG = 16;        // systems per CTA
+// systems per CTA: strided 16 (128-byte row segments); contiguous 8, which
+// fills an SM's threads better (384 rows: 5 CTAs of 192 threads, not 2 of 384)
+template <bool CONTIG>
+constexpr int group_size = CONTIG ? 8 : 16;
 constexpr int MAX_NC = 32;    // chunks of a window
 // exchange values, [chunk][value][system] floats: a neighbour's are a constant
-// distance away, and the two chunks of a warp use all 32 banks
+// distance away, and the chunks of a warp use different banks
 enum { X_E1 = 0, X_S1, X_A0, X_B0, X_B7, X_E2, X_S2, X_COUNT };
 
 // Factors of one chunk as pairs (row k, row k + 8).
@@ -137,15 +140,15 @@ __device__ __forceinline__ void carry_in(float2 (&v)[8], float XB, const F& f) {
 // ---------------------------------------------------------------------------
 // the kernel
 // ---------------------------------------------------------------------------
-// Doubles of the tile: strided [row][16], contiguous [system][Wr + 2].
+// Doubles of the tile: strided [row][16], contiguous [8][Wr + 2].
 template <bool CONTIG>
 __host__ __device__ constexpr size_t tile_elems(int Wr) {
-  return CONTIG ? (size_t)SG * (Wr + 2) : (size_t)SG * Wr;
+  return (size_t)group_size<CONTIG> * (CONTIG ? Wr + 2 : Wr);
 }
 template <bool CONTIG>
 __host__ __device__ constexpr size_t smem_of(int Wr, int nc, int stash_rows) {
-  return 128 + (tile_elems<CONTIG>(Wr) + (size_t)stash_rows * SG) * 8 + (size_t)X_COUNT * nc * SG * 4 +
-         3 * sizeof(Tab) + 16;
+  return 128 + (tile_elems<CONTIG>(Wr) + (size_t)stash_rows * group_size<CONTIG>)*8 +
+         (size_t)X_COUNT * nc * group_size<CONTIG> * 4 + 3 * sizeof(Tab) + 16;
 }
 
 // Untiled bulk copies (both addresses 16-byte aligned, whole 16-byte units).
@@ -172,15 +175,16 @@ __global__ void __launch_bounds__(512, 2)
   // row r of a system: col[r * RS]; contiguous systems lie Wr + 2 doubles
   // apart, so the 16-byte accesses of a quarter-warp (eight systems, the same
   // two rows) touch all 32 banks
+  constexpr int SG = group_size<CONTIG>;
   constexpr int RS = CONTIG ? 1 : SG;
   double* tile = reinterpret_cast<double*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~(uintptr_t)127);
-  double* stash = tile + tile_elems<CONTIG>(g.Wr);  // [H][16], SEQ
+  double* stash = tile + tile_elems<CONTIG>(g.Wr);  // [H][SG], SEQ
   float* xch = reinterpret_cast<float*>(stash + (SEQ ? (size_t)g.H * SG : 0));
   Tab* tabs = reinterpret_cast<Tab*>(xch + (size_t)X_COUNT * g.nc * SG);  // head, tail, interior
   uint64_t* bar = reinterpret_cast<uint64_t*>(tabs + 3);
   const Consts& K = a.k;
   const int t = threadIdx.x, nt = blockDim.x;
-  const int s = t & 15, c = t >> 4;
+  const int s = t & (SG - 1), c = t / SG;
   const int r0 = ROWS * c;
   const int grp = SEQ ? (int)blockIdx.x : (int)(blockIdx.x / g.P);
   const int plane = grp / g.gpp;
@@ -379,8 +383,8 @@ __global__ void __launch_bounds__(512, 2)
     }
 
     // ---- FP32 solve ----
-    const int wp = c >> 1;
-    const bool tab = wp == 0 || wp == last >> 1;  // by warp
+    constexpr int CW = 32 / SG;  // chunks of a warp
+    const bool tab = c / CW == 0 || c / CW == last / CW;
     const bool dead = c > last;                   // rows beyond the system only
     const ByConst fc{K};
     const ByTab ft{tabs + (c == 0 ? 0 : c == last ? 1 : 2)};
@@ -516,22 +520,24 @@ __global__ void __launch_bounds__(512, 2)
     }
     if (!SEQ || ++w == g.P) break;
   }
-  if (__any_sync(__activemask(), rmax >= RANGE_MAG) && (t & 15) == 0 && a.status) atomicOr(a.status, 1u);
+  if (__any_sync(__activemask(), rmax >= RANGE_MAG) && (t & 7) == 0 && a.status) atomicOr(a.status, 1u);
 }
 
 }  // namespace r2n
 
 struct R2N {
+  struct Layout {
+    int H = 0, P = 1, Wr = 0, nc = 0;
+  };
   int n = 0;
-  int H = 0, P = 1, Wr = 0, nc = 0;
+  Layout lay[2];  // strided, contiguous
   bool gen = false;
   int device = 0, sms = 152;
   r2::Args args;
-  r2n::Tables* d_tables = nullptr;
-  unsigned* d_status = nullptr;
+  r2n::Tables* d_tables = nullptr;  // [2]
+  unsigned* d_status = nullptr;     // behind them
   ~R2N() {
     if (d_tables) cudaFree(d_tables);
-    if (d_status) cudaFree(d_status);
   }
 };
 
@@ -580,7 +586,9 @@ int r2n_create(R2N** out, const Plan& p) {
   *out = nullptr;
   const int n = p.n;
   const Matrix& m = p.mat;
-  if (n < 64 || m.nh != 1 || m.nt != 1) return NTK_OK;
+  // (64 rows: the two chunks with tables are half of each system, 64^3 along x
+  // 10.5 us against the chunked kernel's 8.9; from 100 on this one is faster)
+  if (n < 96 || m.nh != 1 || m.nt != 1) return NTK_OK;
   // pivot fixed point of the interior
   double u = m.bi;
   for (int it = 0; it < 4096; ++it) {
@@ -602,28 +610,33 @@ int r2n_create(R2N** out, const Plan& p) {
   int H = 0;
   for (double q = 1.0; q > std::ldexp(1.0, -56); q *= mult) ++H;
   H = (H + 3) & ~1;  // even: window starts stay 16-byte aligned
-  // windows: the fewest rows solved, weighed by the share of the 1024
-  // threads (64 registers each) that whole CTAs of 16 systems can fill
-  double best = 0.0;
-  for (int P = 1; P <= 4096; ++P) {
-    const int Wr = (int)(((long long)n + 2LL * H * (P - 1) + 16 * P - 1) / (16 * P)) * 16;
-    if (P > 1 && Wr < 4 * H + 64) break;  // halos would be half of the work
-    if (Wr > 16 * MAX_NC) continue;
-    const double occ = (double)(1024 / Wr) * Wr / 1024.0;
-    const double cost = (double)P * Wr / (0.3 + 0.7 * occ);
-    if (best == 0.0 || cost < best) {
-      best = cost;
-      r->P = P;
-      r->Wr = Wr;
+  // windows: the fewest rows solved for the share of the 1024 threads (64
+  // registers each) that whole CTAs can fill; several small CTAs overlap their
+  // phases better than two large ones
+  for (int lay = 0; lay < 2; ++lay) {
+    const int sg = lay ? group_size<true> : group_size<false>;
+    R2N::Layout& y = r->lay[lay];
+    double best = 0.0;
+    for (int P = 1; P <= 4096; ++P) {
+      const int Wr = (int)(((long long)n + 2LL * H * (P - 1) + 16 * P - 1) / (16 * P)) * 16;
+      if (P > 1 && Wr < 4 * H + 64) break;  // halos would be half of the work
+      if (Wr > 16 * MAX_NC) continue;
+      const int threads = Wr / 16 * sg, ctas = std::min(1024 / threads, 32);
+      const double cost = (double)P * Wr / (ctas * threads * (1.0 - 0.1 / ctas));
+      if (best == 0.0 || cost < best) {
+        best = cost;
+        y.P = P;
+        y.Wr = Wr;
+      }
+      if (P > 1 && P * (long long)(512 - 2 * H) > 4LL * n) break;
     }
-    if (P > 1 && P * (long long)(512 - 2 * H) > 4LL * n) break;
+    if (best == 0.0) {
+      delete r;
+      return NTK_OK;
+    }
+    y.H = y.P > 1 ? H : 0;
+    y.nc = y.Wr / 16;
   }
-  if (best == 0.0) {
-    delete r;
-    return NTK_OK;
-  }
-  r->H = r->P > 1 ? H : 0;
-  r->nc = r->Wr / 16;
   r->gen = !(r2::pow2_or_zero(m.ai) && r2::pow2_or_zero(m.bi) && r2::pow2_or_zero(m.ci));
   // constants of the interior, and its residual
   r2::Args& a = r->args;
@@ -645,63 +658,61 @@ int r2n_create(R2N** out, const Plan& p) {
   a.nca = r2::splat(-(float)m.ai);
   a.ncb = r2::splat(-(float)m.bi);
   a.ncc = r2::splat(-(float)m.ci);
-  Tables* tb = new (std::nothrow) Tables();
-  if (!tb) {
-    delete r;
-    set_error("out of host memory");
-    return NTK_ERR_ALLOC;
-  }
-  for (int i = 0; i < 8; ++i) {
-    tb->plain.nl[i] = k.nl;
-    tb->plain.g[i] = k.g;
-    tb->plain.nw[i] = k.nw;
-    tb->plain.phi[i] = k.phi[i];
-    tb->plain.psi[i] = k.psi[i];
-  }
-  bool ok = true;
-  for (int kind = 0; kind < KINDS && ok; ++kind) {
-    if ((kind == WHOLE) != (r->P == 1) || (kind == MIDDLE && r->P < 3)) continue;
-    const bool cut_head = kind == MIDDLE || kind == LAST, cut_tail = kind == FIRST || kind == MIDDLE;
-    const int L = r->Wr - 2 * r->H;
-    const int rows = kind == WHOLE ? n : kind == LAST ? n - (r->P - 1) * L : r->Wr;
-    Matrix q;
-    q.n = rows;
-    const double co[7] = {cut_head ? m.bi : m.b(0),     cut_head ? m.ci : m.c(0),     m.ai, m.bi, m.ci,
-                          cut_tail ? m.ai : m.a(n - 1), cut_tail ? m.bi : m.b(n - 1)};
-    q.set_reference(co);
-    std::vector<double> fl, fu, fw(rows);
-    ok = rows >= 48 && rows <= r->Wr && factor_host(q, fl, fu);
-    if (!ok) break;
-    for (int i = 0; i < rows; ++i) fw[i] = q.c(i) / fu[i];
-    // every chunk but the first and the last has the interior's factors
-    const int last = (rows - 1) / 16;
-    for (int i = 16; i < 16 * last && ok; ++i)
-      ok = near(fl[i], l) && near(fu[i], u) && near(fw[i], w);
-    Kind& kd = tb->kind[kind];
-    kd.head = table_of(fl, fu, fw, 0);
-    kd.tail = table_of(fl, fu, fw, 16 * last);
-    for (int e = 0; e < 3; ++e) {
-      kd.hd[e] = r2::to_dwc(e == 0 ? 0.0 : e == 1 ? co[0] : co[1]);
-      kd.td[e] = r2::to_dwc(e == 0 ? co[5] : e == 1 ? co[6] : 0.0);
+  // both layouts' tables and, behind them, the status word
+  std::vector<unsigned char> host(2 * sizeof(Tables) + 16, 0);
+  for (int lay = 0; lay < 2; ++lay) {
+    const R2N::Layout& y = r->lay[lay];
+    Tables tb;
+    std::memset(&tb, 0, sizeof(tb));
+    for (int i = 0; i < 8; ++i) {
+      tb.plain.nl[i] = k.nl;
+      tb.plain.g[i] = k.g;
+      tb.plain.nw[i] = k.nw;
+      tb.plain.phi[i] = k.phi[i];
+      tb.plain.psi[i] = k.psi[i];
     }
-  }
-  if (!ok) {
-    delete tb;
-    delete r;
-    return NTK_OK;
+    bool ok = true;
+    for (int kind = 0; kind < KINDS && ok; ++kind) {
+      if ((kind == WHOLE) != (y.P == 1) || (kind == MIDDLE && y.P < 3)) continue;
+      const bool cut_head = kind == MIDDLE || kind == LAST, cut_tail = kind == FIRST || kind == MIDDLE;
+      const int rows = kind == WHOLE ? n : kind == LAST ? n - (y.P - 1) * (y.Wr - 2 * y.H) : y.Wr;
+      Matrix q;
+      q.n = rows;
+      const double co[7] = {cut_head ? m.bi : m.b(0),     cut_head ? m.ci : m.c(0),     m.ai, m.bi, m.ci,
+                            cut_tail ? m.ai : m.a(n - 1), cut_tail ? m.bi : m.b(n - 1)};
+      q.set_reference(co);
+      std::vector<double> fl, fu, fw(std::max(rows, 0));
+      ok = rows >= 48 && rows <= y.Wr && factor_host(q, fl, fu);
+      if (!ok) break;
+      for (int i = 0; i < rows; ++i) fw[i] = q.c(i) / fu[i];
+      // every chunk but the first and the last has the interior's factors
+      const int last = (rows - 1) / 16;
+      for (int i = 16; i < 16 * last && ok; ++i) ok = near(fl[i], l) && near(fu[i], u) && near(fw[i], w);
+      Kind& kd = tb.kind[kind];
+      kd.head = table_of(fl, fu, fw, 0);
+      kd.tail = table_of(fl, fu, fw, 16 * last);
+      for (int e = 0; e < 3; ++e) {
+        kd.hd[e] = r2::to_dwc(e == 0 ? 0.0 : e == 1 ? co[0] : co[1]);
+        kd.td[e] = r2::to_dwc(e == 0 ? co[5] : e == 1 ? co[6] : 0.0);
+      }
+    }
+    if (!ok) {
+      delete r;
+      return NTK_OK;
+    }
+    std::memcpy(host.data() + lay * sizeof(Tables), &tb, sizeof(tb));
   }
   cudaGetDevice(&r->device);
   cudaDeviceGetAttribute(&r->sms, cudaDevAttrMultiProcessorCount, r->device);
-  int rc = cuda_status(cudaMalloc(&r->d_tables, sizeof(Tables)), "cudaMalloc(window tables)");
+  int rc = cuda_status(cudaMalloc(&r->d_tables, host.size()), "cudaMalloc(window tables)");
   if (!rc)
-    rc = cuda_status(cudaMemcpy(r->d_tables, tb, sizeof(Tables), cudaMemcpyHostToDevice), "cudaMemcpy(window tables)");
-  if (!rc) rc = cuda_status(cudaMalloc(&r->d_status, sizeof(unsigned)), "cudaMalloc(status)");
-  if (!rc) rc = cuda_status(cudaMemset(r->d_status, 0, sizeof(unsigned)), "cudaMemset(status)");
-  delete tb;
+    rc = cuda_status(cudaMemcpy(r->d_tables, host.data(), host.size(), cudaMemcpyHostToDevice),
+                     "cudaMemcpy(window tables)");
   if (rc) {
     delete r;
     return rc;
   }
+  r->d_status = reinterpret_cast<unsigned*>(r->d_tables + 2);
   *out = r;
   return NTK_OK;
 }
@@ -715,13 +726,15 @@ bool r2n_serves(const R2N* r, const double* in, const double* out, const Batch& 
   const long long plane = b.es == 1 ? (ni - 1) * b.is + r->n : (long long)(r->n - 1) * b.es + ni;
   if (b.es == 1 ? b.is < r->n : (b.is != 1 || b.es < ni)) return false;
   if (planes > 1 && b.os < plane) return false;
-  const long long groups = (ni + r2n::SG - 1) / r2n::SG * planes;
-  if (groups * r->P > 0x7fffffffLL) return false;
+  const R2N::Layout& y = r->lay[b.es == 1];
+  const int sg = b.es == 1 ? r2n::group_size<true> : r2n::group_size<false>;
+  const long long groups = (ni + sg - 1) / sg * planes;
+  if (groups * y.P > 0x7fffffffLL) return false;
   const long long extent = (planes - 1) * b.os + plane;
   if (in != out && in < out + extent && out < in + extent) return false;
   // windows in place: all of a system's windows in one CTA
-  if (in == out && r->P > 1) return rp.kind == RHS_IDENTITY && groups >= r->sms;
-  return groups * r->P >= r->sms;
+  if (in == out && y.P > 1) return rp.kind == RHS_IDENTITY && groups >= r->sms;
+  return groups * y.P >= r->sms;
 }
 
 namespace {
@@ -734,7 +747,7 @@ int r2n_launch(const R2N* r, const CUtensorMap& map, const double* in, double* o
   int rc = allow_smem(k, smem, "cudaFuncSetAttribute(r2n_kernel)");
   if (rc) return rc;
   const long long grid = SEQ ? groups : groups * g.P;
-  k<<<(unsigned)grid, r2n::SG * g.nc, smem, st>>>(map, in, out, g, a, r->d_tables);
+  k<<<(unsigned)grid, r2n::group_size<CONTIG> * g.nc, smem, st>>>(map, in, out, g, a, r->d_tables + CONTIG);
   return cuda_status(cudaGetLastError(), "r2n_kernel");
 }
 
@@ -750,15 +763,18 @@ int r2n_gen(const R2N* r, const CUtensorMap& map, const double* in, double* out,
 int r2n_run(R2N* r, const double* in, double* out, const Batch& b, const RhsParams& rp, double s, int prefetch,
             cudaStream_t st) {
   const long long planes = b.nsys > b.ni ? b.nsys / b.ni : 1, ni = b.nsys / planes;
-  const bool contig = b.es == 1, seq = in == out && r->P > 1;
+  const bool contig = b.es == 1;
+  const R2N::Layout& y = r->lay[contig];
+  const bool seq = in == out && y.P > 1;
+  const int sg = contig ? r2n::group_size<true> : r2n::group_size<false>;
   r2n::Geom g;
   g.n = r->n;
-  g.Wr = r->Wr;
-  g.nc = r->nc;
-  g.H = r->H;
-  g.P = r->P;
+  g.Wr = y.Wr;
+  g.nc = y.nc;
+  g.H = y.H;
+  g.P = y.P;
   g.ni = (int)ni;
-  g.gpp = (int)((ni + r2n::SG - 1) / r2n::SG);
+  g.gpp = (int)((ni + sg - 1) / sg);
   g.is = b.is;
   g.os = planes > 1 ? b.os : 0;
   g.es = b.es;
@@ -770,15 +786,15 @@ int r2n_run(R2N* r, const double* in, double* out, const Batch& b, const RhsPara
   CUtensorMap map;
   std::memset(&map, 0, sizeof(map));
   if (!contig && r2::aligned16(in) && b.es % 2 == 0 && (planes == 1 || b.os % 2 == 0)) {
-    g.boxr = r->Wr > 256 ? r->Wr / 2 : r->Wr;
+    g.boxr = y.Wr > 256 ? y.Wr / 2 : y.Wr;
     const cuuint64_t dims[4] = {(cuuint64_t)ni, (cuuint64_t)r->n, (cuuint64_t)planes, 1};
     const long long ps = planes > 1 ? b.os : (long long)b.es * r->n;
     const cuuint64_t strides[3] = {(cuuint64_t)b.es * 8, (cuuint64_t)ps * 8, (cuuint64_t)ps * planes * 8};
-    const cuuint32_t box[4] = {(cuuint32_t)r2n::SG, (cuuint32_t)g.boxr, 1, 1};
+    const cuuint32_t box[4] = {(cuuint32_t)sg, (cuuint32_t)g.boxr, 1, 1};
     int rc = r2::encode(&map, in, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
     if (rc) return rc;
   }
-  if (g.boxr || g.bulk) g.pf = prefetch * r->sms * (1024 / r->Wr) / 2;
+  if (g.boxr || g.bulk) g.pf = prefetch * r->sms * std::min(1024 / (sg * y.nc), 32) / 2;
   r2::Args a = r->args;
   r2::set_scales(&a, rp.kind == RHS_COMPACT ? rp.sigma0 : 1.0, rp.kind == RHS_COMPACT ? rp.sigmaN : 1.0, s);
   a.status = r->d_status;

@@ -8,7 +8,7 @@ namespace ntk {
 struct R2N;
 
 // Tables for a plan's matrix, or *out = null where this solve does not apply
-// (slow decay, a head that converges too slowly, n < 64); an error only where
+// (slow decay, a head that converges too slowly, n < 96); an error only where
 // an allocation or a copy fails.
 int r2n_create(R2N** out, const Plan& p);
 void r2n_destroy(R2N* r);
