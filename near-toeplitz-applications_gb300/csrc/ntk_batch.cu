@@ -38,6 +38,7 @@
 #include "ntk_device.cuh"
 #include "ntk_internal.h"
 #include "ntk_plan.h"
+#include "ntk_soft_f64.cuh"
 
 namespace ntk {
 
@@ -144,7 +145,11 @@ __global__ void __launch_bounds__(128) batch_f64_kernel(double* __restrict__ d, 
 // only in its first Kh rows (the system's head table for the first window,
 // the pivot sequence from a cut for the others, host-tabulated to the exact
 // fixed point), the system's last two rows, padding rows and a cut end (c
-// dropped); the carry responses are the running products of -l and -c/u.
+// dropped); the carry responses are the running products of -l and -c/u,
+// formed once and kept in registers.  The FP64 pipe bounds the kernel: 6
+// instructions a row and the scans' 20 a lane (9 and 20 with the responses
+// formed twice and the division by u as an FP64 product: 4096 systems of 32 ..
+// 8192 rows 178 -> 127 us).
 constexpr int F64W_M = 16;
 constexpr int F64W_LW = 32 * F64W_M;
 constexpr int F64W_PITCH = 32 * (F64W_M + 1) + 1;  // per-warp tile, chunk pitch M + 1
@@ -194,18 +199,22 @@ __device__ __forceinline__ void f64_window(double* work, double* d, const F64Win
   double v[M];
 #pragma unroll
   for (int k = 0; k < M; ++k) v[k] = tile[lane * (M + 1) + k];
+  // f: the running products of -l (then of -c/u), the chunk's responses to
+  // the carry entering it, formed once beside the sweeps and kept for the
+  // carries; y / u is formed on the integer pipes (ntk_soft_f64.cuh)
+  double f[M];
   double l, g, c;
   // ---- forward ----
   f64w_fac(w, pool, r0, l, g, c);
-  double b = -l;
+  f[0] = -l;
 #pragma unroll
   for (int k = 1; k < M; ++k) {
     f64w_fac(w, pool, r0 + k, l, g, c);
     v[k] = fma(-l, v[k - 1], v[k]);
-    b *= -l;
+    f[k] = f[k - 1] * -l;
   }
   {
-    double a = v[M - 1];
+    double a = v[M - 1], b = f[M - 1];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const double ap = __shfl_up_sync(FULL, a, o);
@@ -217,28 +226,26 @@ __device__ __forceinline__ void f64_window(double* work, double* d, const F64Win
     }
     double carry = __shfl_up_sync(FULL, a, 1);
     if (lane == 0) carry = 0.0;
-    f64w_fac(w, pool, r0, l, g, c);
-    double phi = -l;
-    v[0] = fma(phi, carry, v[0]);
 #pragma unroll
-    for (int k = 1; k < M; ++k) {
-      f64w_fac(w, pool, r0 + k, l, g, c);
-      phi *= -l;
-      v[k] = fma(phi, carry, v[k]);
-    }
+    for (int k = 0; k < M; ++k) v[k] = fma(f[k], carry, v[k]);
   }
   // ---- backward ----
-  f64w_fac(w, pool, r0 + M - 1, l, g, c);
-  v[M - 1] *= g;
-  b = -c;
 #pragma unroll
-  for (int k = M - 2; k >= 0; --k) {
+  for (int k = M - 1; k >= 0; --k) {
     f64w_fac(w, pool, r0 + k, l, g, c);
-    v[k] = fma(-c, v[k + 1], v[k] * g);
-    b *= -c;
+    const SoftFactor sg = soft_factor(g);
+    double y = soft_product(v[k], sg);
+    if (!soft_in_range(v[k], sg)) y = rare_mul(v[k], g);
+    if (k == M - 1) {
+      v[k] = y;
+      f[k] = -c;
+    } else {
+      v[k] = fma(-c, v[(k + 1) % M], y);
+      f[k] = f[(k + 1) % M] * -c;
+    }
   }
   {
-    double a = v[0];
+    double a = v[0], b = f[0];
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const double ap = __shfl_down_sync(FULL, a, o);
@@ -250,15 +257,8 @@ __device__ __forceinline__ void f64_window(double* work, double* d, const F64Win
     }
     double carry = __shfl_down_sync(FULL, a, 1);
     if (lane == 31) carry = 0.0;
-    f64w_fac(w, pool, r0 + M - 1, l, g, c);
-    double psi = -c;
-    v[M - 1] = fma(psi, carry, v[M - 1]);
 #pragma unroll
-    for (int k = M - 2; k >= 0; --k) {
-      f64w_fac(w, pool, r0 + k, l, g, c);
-      psi *= -c;
-      v[k] = fma(psi, carry, v[k]);
-    }
+    for (int k = M - 1; k >= 0; --k) v[k] = fma(f[k], carry, v[k]);
   }
   // ---- central rows back through the tile (coalesced) ----
   __syncwarp();

@@ -36,9 +36,13 @@ struct SoftFactor {
   uint32_t lim;
 };
 
-inline SoftFactor soft_factor(double g) {
+SOFT_HD SoftFactor soft_factor(double g) {
+#ifdef __CUDA_ARCH__
+  const uint64_t u = (uint64_t)__double_as_longlong(g);
+#else
   uint64_t u;
   std::memcpy(&u, &g, 8);
+#endif
   const int e = (int)((u >> 52) & 0x7ff) - 1023;
   SoftFactor f;
   f.mant = (u << 11) | (1ull << 63);
