@@ -124,9 +124,12 @@ int Plan::g_table(double s, const double** out) {
     return NTK_ERR_UNSUPPORTED;
   }
   const size_t rows = chunk.g_offset(n);
-  std::vector<double> g(rows + chunk.g_elems());
+  const size_t soft = rows + ((chunk.g_elems() + 1) & ~(size_t)1);  // g[n] prepared, 16-byte aligned
+  std::vector<double> g(soft + 2 * (size_t)n);
   for (int i = 0; i < n; ++i) g[i] = s / lu_u[i];
   chunk.g_rows(g.data(), g.data() + rows);
+  SoftFactor* sg = reinterpret_cast<SoftFactor*>(g.data() + soft);
+  for (int i = 0; i < n; ++i) sg[i] = soft_factor(g[i]);
   double* d = nullptr;
   int rc = cuda_status(cudaMalloc(&d, sizeof(double) * g.size()), "cudaMalloc(g table)");
   if (rc) return rc;
@@ -138,6 +141,15 @@ int Plan::g_table(double s, const double** out) {
   g_by_scale[s] = d;
   *out = d;
   return NTK_OK;
+}
+
+int Plan::tables(double s, TablesF64* t) {
+  t->l = d_lw;
+  t->w = d_lw + n;
+  const int rc = g_table(s, &t->g);
+  if (!rc)
+    t->sg = reinterpret_cast<const SoftFactor*>(t->g + chunk.g_offset(n) + ((chunk.g_elems() + 1) & ~(size_t)1));
+  return rc;
 }
 
 int Plan::check_device() const {
@@ -156,10 +168,7 @@ int Plan::run(const double* in, double* out, const Batch& b, RhsParams rp, doubl
   if (b.nsys == 0) return NTK_OK;
   if (precision == NTK_FP64) {
     TablesF64 t;
-    t.l = d_lw;
-    t.w = d_lw + n;
-    rc = g_table(s, &t.g);
-    if (rc) return rc;
+    if ((rc = tables(s, &t))) return rc;
     int S = 0;
     if (const ChunkF64::Cfg* cfg = chunk_f64_pick(chunk, b, rp.kind, &S))
       return launch_chunk_f64(chunk, *cfg, S, in, out, b, rp, t, stream);
@@ -173,9 +182,7 @@ int Plan::run_chunks(const double* in, double* out, const Batch& b, const RhsPar
   int rc = check_device();
   if (rc || b.nsys == 0) return rc;
   TablesF64 t;
-  t.l = d_lw;
-  t.w = d_lw + n;
-  if ((rc = g_table(s, &t.g))) return rc;
+  if ((rc = tables(s, &t))) return rc;
   int S = 0;
   const ChunkF64::Cfg* cfg = chunk_f64_pick(chunk, b, rp.kind, &S, true);
   if (!cfg) {

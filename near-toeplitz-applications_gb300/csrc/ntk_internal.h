@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "../../include/ntk.h"
+#include "ntk_soft_f64.cuh"
 
 namespace ntk {
 
@@ -108,6 +109,7 @@ struct TablesF64 {
   const double* l = nullptr;  // l_i = a_i / u_{i-1}
   const double* g = nullptr;  // g_i = s / u_i
   const double* w = nullptr;  // w_i = c_i / u_i
+  const SoftFactor* sg = nullptr;  // g_i prepared for soft_product (Plan::tables)
 };
 
 void set_error(const char* fmt, ...);

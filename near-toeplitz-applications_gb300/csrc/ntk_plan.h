@@ -93,6 +93,7 @@ struct Plan {
   int init(int n, long long nrhs, const double co[7], int precision, int sweeps);
   ~Plan();
   int g_table(double s, const double** out);
+  int tables(double s, TablesF64* t);  // l, w and the g table of scale s
   int check_device() const;
   int run(const double* in, double* out, const Batch& b, RhsParams rp, double s, cudaStream_t stream);
 

@@ -168,11 +168,28 @@ __device__ __forceinline__ double forward_compact(const double* src, double* dst
 
 // ----------------------------------------------------------------------------
 // backward sweep: x_i = g_i eta_i - w_i x_{i+1}, eta read back from dst.
+// g eta runs on the integer pipes (ntk_soft_f64.cuh), PF rows at a time with
+// one range check, which leaves one FP64 instruction a row.
 // ----------------------------------------------------------------------------
+// y[k] = g_{i0 - k} e[k], k < PF
+__device__ __forceinline__ void scaled_rows(const TablesF64& t, int i0, const double (&e)[PF], double (&y)[PF]) {
+  bool in_range = true;
+#pragma unroll
+  for (int k = 0; k < PF; ++k) {
+    const uint4 q = __ldg(reinterpret_cast<const uint4*>(t.sg) + (i0 - k));
+    const SoftFactor f{(uint64_t)q.y << 32 | q.x, q.z, q.w};
+    in_range = in_range && soft_in_range(e[k], f);
+    y[k] = soft_product(e[k], f);
+  }
+  if (!in_range) {
+#pragma unroll
+    for (int k = 0; k < PF; ++k) y[k] = rare_mul(e[k], __ldg(t.g + (i0 - k)));
+  }
+}
+
 template <bool VEC>
-__device__ __forceinline__ void backward(double* dst, long long es, int n, double eta_last,
-                                         const double* __restrict__ g, const double* __restrict__ w) {
-  double x = __ldg(g + (n - 1)) * eta_last;
+__device__ __forceinline__ void backward(double* dst, long long es, int n, double eta_last, const TablesF64& t) {
+  double x = __ldg(t.g + (n - 1)) * eta_last;
   dst[(long long)(n - 1) * es] = x;
   // descending prefetch ring over rows n-2 ... 0
   double ring[PF];
@@ -181,26 +198,25 @@ __device__ __forceinline__ void backward(double* dst, long long es, int n, doubl
     const int i = n - 2 - k;
     if (i >= 0) ring[k] = dst[(long long)i * es];
   }
-  int r0 = 0;  // ring position of row n-2-r0
-  for (; r0 + PF <= n - 1; r0 += PF) {
+  int i = n - 2;  // ring[k]: row i - k
+  for (; i >= PF - 1; i -= PF) {
+    double y[PF];
+    scaled_rows(t, i, ring, y);
+#pragma unroll
+    for (int k = 0; k < PF; ++k)
+      if (i - k - PF >= 0) ring[k] = dst[(long long)(i - k - PF) * es];
 #pragma unroll
     for (int k = 0; k < PF; ++k) {
-      const int i = n - 2 - (r0 + k);
-      const double e = ring[k];
-      const int ip = i - PF;
-      if (ip >= 0) ring[k] = dst[(long long)ip * es];
-      x = fma(-__ldg(w + i), x, __ldg(g + i) * e);
-      dst[(long long)i * es] = x;
+      x = fma(-__ldg(t.w + (i - k)), x, y[k]);
+      dst[(long long)(i - k) * es] = x;
     }
   }
 #pragma unroll
-  for (int k = 0; k < PF; ++k) {
-    const int i = n - 2 - (r0 + k);
-    if (i >= 0) {
-      x = fma(-__ldg(w + i), x, __ldg(g + i) * ring[k]);
-      dst[(long long)i * es] = x;
+  for (int k = 0; k < PF; ++k)
+    if (i - k >= 0) {
+      x = fma(-__ldg(t.w + (i - k)), x, __ldg(t.g + (i - k)) * ring[k]);
+      dst[(long long)(i - k) * es] = x;
     }
-  }
 }
 
 template <int RHS, bool VEC>
@@ -224,7 +240,7 @@ __global__ void __launch_bounds__(128) thomas_f64_kernel(const double* in, doubl
     eta = fma(-__ldg(t.l + (n - 1)), eta, rp.sigmaN * ((-5.0 * fl2 + 4.0 * fl1) + fl0));
     dst[(long long)(n - 1) * b.es] = eta;
   }
-  backward<VEC>(dst, b.es, n, eta, t.g, t.w);
+  backward<VEC>(dst, b.es, n, eta, t);
 }
 
 // ----------------------------------------------------------------------------
@@ -541,11 +557,20 @@ __global__ void __launch_bounds__(32 * XWARPS) thomas_f64_xpose_kernel(const dou
     __syncwarp();
     const int row0 = c * XT;
     const int rows = min(XT, n - row0);
-#pragma unroll 8
-    for (int k = rows - 1; k >= 0; --k) {
-      const int i = row0 + k;
-      const double e = cur[k * XP + lane];
-      x = fma(-__ldg(t.w + i), x, __ldg(t.g + i) * e);
+    int k = rows - 1;
+    for (; k >= PF - 1; k -= PF) {
+      double e[PF], y[PF];
+#pragma unroll
+      for (int q = 0; q < PF; ++q) e[q] = cur[(k - q) * XP + lane];
+      scaled_rows(t, row0 + k, e, y);
+#pragma unroll
+      for (int q = 0; q < PF; ++q) {
+        x = fma(-__ldg(t.w + (row0 + k - q)), x, y[q]);
+        cur[(k - q) * XP + lane] = x;
+      }
+    }
+    for (; k >= 0; --k) {
+      x = fma(-__ldg(t.w + (row0 + k)), x, __ldg(t.g + (row0 + k)) * cur[k * XP + lane]);
       cur[k * XP + lane] = x;
     }
     __syncwarp();
