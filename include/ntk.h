@@ -198,8 +198,10 @@ typedef struct ntk_adi ntk_adi;
 /* Builds the ADI solver for N x N fields (N >= 4).  precision:
  *   NTK_FP64         FP64 over overlapping 32M-row windows, one warp per
  *                    window (halos exact to FP64 rounding), when N >= 128 and
- *                    the factors decay fast enough; otherwise segmented FP64
- *                    sweeps with an N x N FP64 work array.
+ *                    the factors decay fast enough; otherwise whole systems,
+ *                    several threads each, in shared memory (N >= 20), or
+ *                    segmented FP64 sweeps with an N x N FP64 work array
+ *                    where a system does not fit.
  *   NTK_FP32_REFINE  FP32 solve + one double-word refinement sweep per half
  *                    step, over overlapping 32M-row windows (M = 16, 8 or 4;
  *                    needs N >= 128, else NTK_ERR_UNSUPPORTED); matches the
@@ -222,8 +224,8 @@ int ntk_adi_status(ntk_adi* adi, int* flags, void* stream);
 /* The segmentation the plan chose: for windows (NTK_FP32, NTK_FP32_REFINE,
  * and NTK_FP64 where they apply) the windows' central rows, halo and windows
  * per system; for the partitioned FP32 solve 512, 0 and the partitions per
- * system; for the segmented FP64 sweeps segment length, halo and segments
- * per system (1 segment = plain sweeps). */
+ * system; for whole FP64 systems N, 0 and 1; for the segmented FP64 sweeps
+ * segment length, halo and segments per system (1 segment = plain sweeps). */
 int ntk_adi_segments(const ntk_adi* adi, int* seg_len, int* halo, int* nseg);
 
 /* One time step on device arrays u, d_x, d_y (N x N, C order), with the

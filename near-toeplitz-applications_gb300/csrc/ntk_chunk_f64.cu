@@ -433,12 +433,13 @@ void ChunkF64::g_rows(const double* g, double* out) const {
 // SM's share, plus twice the length of one CTA's dependent chain (the first
 // CTAs fill the pipe and the last ones drain it; more where a second wave
 // starts late); row segments of strided systems below 128 bytes cost up to an
-// eighth.  One thread per system: n (3 + extra) instructions a warp times the
+// eighth.  One thread per system: n (2 + extra) instructions a warp times the
 // measured distance from the pipe's rate, which falls as more warps hide each
-// other's loads.  Measured, us, one thread a system against chunks: 512 rows
-// contiguous, 4096 systems 161 : 23, 16384 163 : 75, 65536 291 : 273, compact
-// with 262144 1169 : 1272; strided compact, 13472 systems of 333 rows 79 : 56,
-// 79990 240 : 275.
+// other's loads (contiguous systems, whose tiles take most of the time: as
+// measured with one instruction more).  Measured, us, one thread a system
+// against chunks: 512 rows contiguous, 4096 systems 161 : 23, 16384 163 : 75,
+// 65536 291 : 273, compact with 262144 1143 : 1272; strided compact, 13472
+// systems of 333 rows 79 : 56, 79990 207 : 275.
 const ChunkF64::Cfg* chunk_f64_pick(const ChunkF64& c, const Batch& b, int rhs, int* S, bool always) {
   const bool strided = b.es != 1;
   const int extra = rhs == RHS_COMPACT ? 1 : 0;
@@ -463,8 +464,8 @@ const ChunkF64::Cfg* chunk_f64_pick(const ChunkF64& c, const Batch& b, int rhs, 
     }
   if (always) return best;
   const double load = std::ceil((double)((b.nsys + 31) / 32) / (4 * SMS));
-  const double far = strided ? 0.97 + 0.55 / load : 0.95 + 1.5 / load;
-  return best && best_cost < load * c.n * (3 + extra) * far ? best : nullptr;
+  const double plain = strided ? (2 + extra) * (0.92 + 1.2 / load) : (3 + extra) * (0.95 + 1.5 / load);
+  return best && best_cost < load * c.n * plain ? best : nullptr;
 }
 
 int launch_chunk_f64(const ChunkF64& cf, const ChunkF64::Cfg& cfg, int S, const double* in, double* out,

@@ -13,16 +13,20 @@
 // and each thread runs the Thomas recurrences on one system:
 //   forward   eta_i = D_i - l_i * eta_{i-1}          (1 DFMA; +1 DADD for the
 //                                                      compact RHS difference)
-//   backward  x_i  = g_i * eta_i - w_i * x_{i+1}     (1 DMUL off the chain + 1 DFMA)
-// i.e. 3 (in-place solve) or 4 (fused compact derivative) FP64 instructions
+//   backward  x_i  = g_i * eta_i - w_i * x_{i+1}     (1 DFMA; g_i eta_i off the
+//                                                      chain, on the integer pipes)
+// i.e. 2 (in-place solve) or 3 (fused compact derivative) FP64 instructions
 // per unknown, against ~10 plus two FP64 divisions per unknown in the
 // reference's cyclic reduction.  Nothing else may touch the FP64 pipe in the
 // row loops: a condition on the row (first, last) around FP64 work becomes
 // predicated instructions there, which hold the pipe like executed ones, so
 // the end rows are handled outside (512^3 derivatives: x 1446 -> 1169 us, y
-// 1157 -> 1030 us, 4 instructions a row alone 1033 us).  The forward values eta are parked in the
-// output array (they are L2-resident until the backward pass overwrites them
-// with x), so no shared memory is needed and occupancy is set by registers.
+// 1157 -> 1030 us; with g eta on the integer pipes 1143 and 833 us).  The
+// forward values eta are parked in the output array: many more systems are in
+// flight than the L2 holds, so the backward sweep of y and z reads them from
+// HBM (29 B per row in all) and the FP64 pipe and HBM bound one sweep each; x
+// is held back by its transposing tiles (tiles of 8 rows, rings of 4, CTAs of 2
+// and 8 warps measured within 5%).
 // Threads of a warp take adjacent systems: for y/z sweeps of a 3D field these
 // are adjacent x-columns, so every row access is one coalesced 256-byte
 // segment and no permute pass is needed.
