@@ -5,19 +5,21 @@
 // 2048 x 2048 one 2046: 8 and 64 warps for 152 SMs, each walking 2 n
 // dependent rows through global memory.  Here a CTA keeps S whole systems in
 // shared memory and gives every system T threads of C consecutive rows:
-//   forward   y_i = d_i - l_i y_{i-1} over the chunk from zero, in place;
-//             the chunks' carries are an exact affine scan over the T chunk
-//             ends (log2 T steps through shared memory, the products of the
-//             multipliers tabulated on the host: one FMA a step)
-//   backward  y_i = y'_i + phi_i y_{s-1}, x_i = g_i y_i - (c_i / u_i) x_{i+1}
-//             from zero, then the same scan from the other end
-//   last      x_i = x'_i + psi_i x_{e+1}, stored
-// (phi, psi: the responses of a chunk's sweeps to the carry entering it, as
-// in ntk_adi_f64.cu.)  Nothing is truncated, so any matrix that factors is
-// served, at 5 operations a row (+1 for the compact difference)
-// against 3 (+1): the FP64 pipe (one warp instruction per ~73 clocks and
-// sub-partition) bounds both kernels, and this one wins where one thread per
-// system leaves the pipe idle (chunk_f64_pick).
+//   forward   y_i = d_i - l_i y_{i-1} over the chunk from zero, for its end
+//             value only; the chunks' carries are an exact affine scan over the
+//             T ends (log2 T steps through shared memory, the products of the
+//             multipliers tabulated on the host: one FMA a step); then the
+//             sweep again from the carry, in place
+//   backward  x_i = g_i y_i - (c_i / u_i) x_{i+1} likewise from the other end,
+//             the second time straight to the results
+// Sweeping twice costs an FMA a row, as adding the carries' responses to the
+// rows of one sweep would, and rounds as the sequential sweeps do (2046 systems
+// of 2048 rows: error against 64 bits 1.07e-16, with added responses 1.34e-16;
+// 1 - 7% slower).  Nothing is truncated, so any matrix that factors is served,
+// at 5 operations a row (+1 for the compact difference) against 3 (+1): the
+// FP64 pipe (one warp instruction per ~76 clocks and sub-partition) bounds both
+// kernels, and this one wins where one thread per system leaves the pipe idle
+// (chunk_f64_pick).
 // Rows stay in shared memory between the sweeps, not in registers, so a
 // chunk may be long: the scans' 2 log2 T instructions a thread are spread
 // over C rows.  A contiguous system's chunks lie C + 1 doubles apart (odd: the
@@ -30,7 +32,7 @@
 // tail), so the factors stay in L1.
 // Measured, one thread per system against this kernel: 2046 systems of 2048
 // rows 754 -> 45 us (67 with g y on the FP64 pipe; the pipe alone: 34 us),
-// compact derivative of a 256 x 256 field 97 -> 11.5 us (most of it the call).
+// compact derivative of a 256 x 256 field 97 -> 8.2 us (most of it the call).
 // A system with a value that is not finite, or that overflows on the way, is
 // solved again row by row from its input, so that inf and nan spread exactly
 // as in the one-thread sweeps.
@@ -51,7 +53,7 @@ constexpr int RB = 4;  // rows per batch of a sweep: their loads are issued ahea
 struct ChunkParams {
   int n, S, T, C, P, steps, shift;  // P: pitch of a contiguous system; shift: log2 S (strided) or log2 T
   unsigned invC;       // ceil(2^32 / C): r / C = umulhi(r, invC) for the rows of a system
-  const double* tab;      // [ncls][4][C]: -l, phi, -w, psi
+  const double* tab;      // [ncls][2][C]: -l, -w
   const double* g;        // [ncls][C]
   const SoftFactor* sg;   // the same, prepared
   const double* scan;  // [2][steps][T]
@@ -155,14 +157,13 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
   const int len = on ? max(0, min(c.C, c.n - r0)) : 0;
   double* row = col + (STRIDED ? r0 * c.S : t * (c.C + 1));  // row r0 + k: row[k * rs]
   const int cls = __ldg(c.cls + t);
-  const double* ml = c.tab + (size_t)cls * 4 * c.C;
-  const double* phi = ml + c.C;
-  const double* mw = phi + c.C;
-  const double* psi = mw + c.C;
+  const double* ml = c.tab + (size_t)cls * 2 * c.C;
+  const double* mw = ml + c.C;
   const double* g = c.g + (size_t)cls * c.C;
   const SoftFactor* sg = c.sg + (size_t)cls * c.C;
 
-  // ---- forward over the chunk from zero ----
+  // ---- forward over the chunk from zero, for its end value only (the compact
+  // difference is left in the rows) ----
   double y = 0.0;
   {
     // the neighbours' edge rows, and the end rows' one-sided stencils
@@ -198,9 +199,9 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
             d = fn - fm;
             fm = v[q];
             if (r0 + k + q == 0 || r0 + k + q == c.n - 1) d = be;
+            row[(k + q) * rs] = d;
           }
           y = fma(m[q], y, d);
-          row[(k + q) * rs] = y;
         }
       }
 #pragma unroll
@@ -221,7 +222,30 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
   __syncthreads();
   const double cin = t > 0 ? ex[cur * nt + tid - xs] : 0.0;
 
-  // ---- backward over the chunk from zero ----
+  // ---- forward again from the carry ----
+  {
+    double z = cin, v[RB];
+#pragma unroll
+    for (int q = 0; q < RB; ++q) v[q] = q < len ? row[q * rs] : 0.0;
+    for (int k = 0; k < len; k += RB) {
+      double nx[RB], m[RB];
+#pragma unroll
+      for (int q = 0; q < RB; ++q) {
+        nx[q] = k + RB + q < len ? row[(k + RB + q) * rs] : 0.0;
+        m[q] = __ldg(ml + k + q);
+      }
+#pragma unroll
+      for (int q = 0; q < RB; ++q)
+        if (k + q < len) {
+          z = fma(m[q], z, v[q]);
+          row[(k + q) * rs] = z;
+        }
+#pragma unroll
+      for (int q = 0; q < RB; ++q) v[q] = nx[q];
+    }
+  }
+  // ---- backward over the chunk from zero, for its start value; the rows keep
+  // g y ----
   double x = 0.0;
   {
     const int k0 = (len - 1) & ~(RB - 1);
@@ -239,7 +263,6 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
       }
 #pragma unroll
       for (int q = 0; q < RB; ++q) {
-        v[q] = fma(__ldg(phi + k + q), cin, v[q]);
         in_range = in_range && (k + q >= len || soft_in_range(v[q], f[q]));
         gy[q] = soft_product(v[q], f[q]);
       }
@@ -251,7 +274,7 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
       for (int q = RB - 1; q >= 0; --q)
         if (k + q < len) {
           x = fma(__ldg(mw + k + q), x, gy[q]);
-          row[(k + q) * rs] = x;
+          row[(k + q) * rs] = gy[q];
         }
 #pragma unroll
       for (int q = 0; q < RB; ++q) v[q] = nx[q];
@@ -273,16 +296,32 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
   // whatever is not finite anywhere in the system has reached row 0
   const bool ok = finite(ex[cur * nt + tid - t * xs]);
 
-  // ---- carries into the chunk, results out ----
-  if (STRIDED) {
-    if (on && ok) {
-      double* dst = out + base + (long long)r0 * b.es;
-#pragma unroll 4
-      for (int k = 0; k < len; ++k) dst[(long long)k * b.es] = fma(__ldg(psi + k), xin, row[k * rs]);
+  // ---- backward again from the carry, results out ----
+  {
+    double* dst = out + base + (long long)r0 * b.es;
+    const int k0 = (len - 1) & ~(RB - 1);
+    double z = xin, v[RB];
+#pragma unroll
+    for (int q = 0; q < RB; ++q) v[q] = len > 0 && k0 + q < len ? row[(k0 + q) * rs] : 0.0;
+    for (int k = k0; k >= 0; k -= RB) {
+      double nx[RB], m[RB];
+#pragma unroll
+      for (int q = 0; q < RB; ++q) {
+        nx[q] = k >= RB ? row[(k - RB + q) * rs] : 0.0;
+        m[q] = __ldg(mw + k + q);
+      }
+#pragma unroll
+      for (int q = RB - 1; q >= 0; --q)
+        if (k + q < len) {
+          z = fma(m[q], z, v[q]);
+          if (!STRIDED) row[k + q] = z;
+          else if (ok) dst[(long long)(k + q) * b.es] = z;
+        }
+#pragma unroll
+      for (int q = 0; q < RB; ++q) v[q] = nx[q];
     }
-  } else {
-#pragma unroll 4
-    for (int k = 0; k < len; ++k) row[k] = fma(__ldg(psi + k), xin, row[k]);
+  }
+  if (!STRIDED) {
     __syncthreads();
     if (on && ok) {
       double* dst = out + base;
@@ -357,22 +396,17 @@ int ChunkF64::init(int n_, const double* l, const double* u, const double* w) {
         f.rep.push_back(t);
         // its columns; rows past the system's end hold zeros
         const size_t at = tab.size();
-        tab.resize(at + 4 * (size_t)f.C, 0.0);
+        tab.resize(at + 2 * (size_t)f.C, 0.0);
         double* q = tab.data() + at;
-        double p = 1.0;
+        double pl = 1.0, pw = 1.0;  // the responses of its end (start) to the carry entering it
         for (int k = 0; k < len; ++k) {
           q[k] = -l[r0 + k];
-          p *= -l[r0 + k];
-          q[f.C + k] = p;
-          q[2 * f.C + k] = -w[r0 + k];
+          q[f.C + k] = -w[r0 + k];
+          pl *= q[k];
         }
-        Phi[t] = len ? p : 0.0;
-        p = 1.0;
-        for (int k = len - 1; k >= 0; --k) {
-          p *= -w[r0 + k];
-          q[3 * f.C + k] = p;
-        }
-        Psi[t] = len ? p : 0.0;
+        for (int k = len - 1; k >= 0; --k) pw *= q[f.C + k];
+        Phi[t] = len ? pl : 0.0;
+        Psi[t] = len ? pw : 0.0;
       } else {
         Phi[t] = Phi[f.rep[id]];
         Psi[t] = Psi[f.rep[id]];
