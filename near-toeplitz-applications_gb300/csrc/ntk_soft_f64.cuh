@@ -4,13 +4,20 @@
 // ~76 clocks, while its integer and FP32 pipes idle: an FP64 operation that
 // takes fewer than 76 issue slots in integer arithmetic, off the dependent
 // chain, is cheaper there, and runs beside the FP64 instructions that stay.
-// soft_product (41 clocks) is such an operation: the exact 106-bit product's upper 64 bits,
-// rounded to 53, i.e. the IEEE product except that a result within 2^-62 of a
-// rounding boundary may round to its other neighbour.  Operands outside the
-// range where neither overflow nor underflow can occur (zero, subnormal, inf
-// and nan among them) take the FP64 pipe's product.
-// Compiles for the host too, where tests/soft_f64_check.cpp compares it with
-// the host's IEEE product.
+// soft_product (~45 clocks) is such an operation: the exact 106-bit product
+// rounded to 53 bits, ties to even, i.e. the IEEE product bit for bit.  Ties
+// are common where an operand is short (one product in six for 1.5 or 0.75).
+// Operands outside the range where neither overflow nor underflow can occur
+// (zero, subnormal, inf and nan among them) take the FP64 pipe's product.
+// soft_product_untied (41 clocks) rounds half up and serves operands whose
+// product cannot be a tie; the one-thread sweeps, which both pipes bound, take
+// it and leave the others to the FP64 pipe (a 512^3 gradient 2817 -> 2919 us
+// with soft_product, 2836 so).  Kernels with few rows a thread take
+// soft_product: a block of rows with a boundary value of 1 or a factor of 1.5
+// beside the FP64 product costs them more (a 256 x 256 derivative 8.2 -> 10.2
+// us, ADI steps 5%).
+// Compiles for the host too, where tests/soft_f64_check.cpp and
+// tests/soft_f64_ties.cpp compare it with the host's IEEE product.
 #pragma once
 #include <cstdint>
 #include <cstring>
@@ -36,19 +43,51 @@ struct SoftFactor {
   uint32_t lim;
 };
 
-SOFT_HD SoftFactor soft_factor(double g) {
+SOFT_HD uint32_t soft_hi(double a) {
 #ifdef __CUDA_ARCH__
-  const uint64_t u = (uint64_t)__double_as_longlong(g);
+  return (uint32_t)__double2hiint(a);
 #else
   uint64_t u;
-  std::memcpy(&u, &g, 8);
+  std::memcpy(&u, &a, 8);
+  return (uint32_t)(u >> 32);
 #endif
+}
+SOFT_HD uint32_t soft_lo(double a) {
+#ifdef __CUDA_ARCH__
+  return (uint32_t)__double2loint(a);
+#else
+  uint64_t u;
+  std::memcpy(&u, &a, 8);
+  return (uint32_t)u;
+#endif
+}
+SOFT_HD double soft_double(uint64_t r) {
+#ifdef __CUDA_ARCH__
+  return __longlong_as_double((long long)r);
+#else
+  double x;
+  std::memcpy(&x, &r, 8);
+  return x;
+#endif
+}
+
+SOFT_HD SoftFactor soft_factor(double g) {
+  const uint64_t u = (uint64_t)soft_hi(g) << 32 | soft_lo(g);
   const int e = (int)((u >> 52) & 0x7ff) - 1023;
   SoftFactor f;
   f.mant = (u << 11) | (1ull << 63);
   // the leading one of the rounded mantissa adds one to the exponent field
   f.eadd = ((uint32_t)e << 20) + (uint32_t)(u >> 63 << 31);
   f.lim = (e >= -60 && e <= 60) ? (1980u - 64u) << 20 : 0u;
+  return f;
+}
+
+// The factor for soft_product_untied: factors of 2 .. 33 significant bits are
+// not served (a product by one of 34 or more bits is no tie unless the
+// operand's lower word is zero, a product by a power of two is exact).
+SOFT_HD SoftFactor soft_factor_untied(double g) {
+  SoftFactor f = soft_factor(g);
+  if ((f.mant & 0x7fffffffull) == 0 && f.mant << 1 != 0) f.lim = 0;
   return f;
 }
 
@@ -75,25 +114,35 @@ static __device__ __noinline__ double one_sided(double sigma, double f0, double 
 
 // whether soft_product serves operand a
 SOFT_HD bool soft_in_range(double a, const SoftFactor& f) {
-#ifdef __CUDA_ARCH__
-  const uint32_t ah = (uint32_t)__double2hiint(a);
-#else
-  uint64_t ua;
-  std::memcpy(&ua, &a, 8);
-  const uint32_t ah = (uint32_t)(ua >> 32);
-#endif
-  return (ah & 0x7fffffffu) - (64u << 20) < f.lim;
+  return (soft_hi(a) & 0x7fffffffu) - (64u << 20) < f.lim;
 }
 
 // a times the factor, a in range
 SOFT_HD double soft_product(double a, const SoftFactor& f) {
-#ifdef __CUDA_ARCH__
-  const uint32_t ah = (uint32_t)__double2hiint(a), al = (uint32_t)__double2loint(a);
-#else
-  uint64_t ua;
-  std::memcpy(&ua, &a, 8);
-  const uint32_t ah = (uint32_t)(ua >> 32), al = (uint32_t)ua;
-#endif
+  const uint32_t ah = soft_hi(a), al = soft_lo(a);
+  const uint32_t mh = (ah << 11 | al >> 21) | 0x80000000u, ml = al << 11;
+  const uint32_t gh = (uint32_t)(f.mant >> 32), gl = (uint32_t)f.mant;
+  // the 128-bit product: t, and its lower words as a sticky word
+  const uint64_t p = (uint64_t)ml * gl;
+  const uint64_t q = (uint64_t)mh * gl + (p >> 32);
+  const uint64_t s = (uint64_t)ml * gh + (uint32_t)q;
+  uint64_t t = (uint64_t)mh * gh + (q >> 32) + (s >> 32);  // [2^62, 2^64)
+  const uint32_t low = (uint32_t)s | (uint32_t)p;
+  uint32_t e = (ah & 0xfff00000u) + f.eadd;
+  if (t >> 63 == 0) {
+    t <<= 1;
+    e -= 1u << 20;
+  }
+  uint64_t r = ((uint64_t)e << 32) + (t >> 11) + ((t >> 10) & 1u);
+  if (((((uint32_t)t ^ 0x400u) & 0x7ffu) | low) == 0) r &= ~(uint64_t)1;  // a tie, rounded up: the even neighbour
+  return soft_double(r);
+}
+
+// whether soft_product_untied is the IEEE product of a and a soft_factor_untied
+SOFT_HD bool soft_untied(double a, const SoftFactor& f) { return soft_in_range(a, f) && soft_lo(a) != 0; }
+
+SOFT_HD double soft_product_untied(double a, const SoftFactor& f) {
+  const uint32_t ah = soft_hi(a), al = soft_lo(a);
   const uint64_t m = (((uint64_t)ah << 32 | al) << 11) | (1ull << 63);
   uint64_t t = soft_umul64hi(m, f.mant);  // [2^62, 2^64)
   uint32_t e = (ah & 0xfff00000u) + f.eadd;
@@ -101,14 +150,7 @@ SOFT_HD double soft_product(double a, const SoftFactor& f) {
     t <<= 1;
     e -= 1u << 20;
   }
-  const uint64_t r = ((uint64_t)e << 32) + (t >> 11) + ((t >> 10) & 1u);
-#ifdef __CUDA_ARCH__
-  return __longlong_as_double((long long)r);
-#else
-  double x;
-  std::memcpy(&x, &r, 8);
-  return x;
-#endif
+  return soft_double(((uint64_t)e << 32) + (t >> 11) + ((t >> 10) & 1u));
 }
 
 }  // namespace ntk

@@ -182,8 +182,8 @@ __device__ __forceinline__ void scaled_rows(const TablesF64& t, int i0, const do
   for (int k = 0; k < PF; ++k) {
     const uint4 q = __ldg(reinterpret_cast<const uint4*>(t.sg) + (i0 - k));
     const SoftFactor f{(uint64_t)q.y << 32 | q.x, q.z, q.w};
-    in_range = in_range && soft_in_range(e[k], f);
-    y[k] = soft_product(e[k], f);
+    in_range = in_range && soft_untied(e[k], f);
+    y[k] = soft_product_untied(e[k], f);
   }
   if (!in_range) {
 #pragma unroll
