@@ -34,8 +34,10 @@
 // rows 754 -> 45 us (67 with g y on the FP64 pipe; the pipe alone: 34 us),
 // compact derivative of a 256 x 256 field 97 -> 8.2 us (most of it the call).
 // A system with a value that is not finite, or that overflows on the way, is
-// solved again row by row from its input, so that inf and nan spread exactly
-// as in the one-thread sweeps.
+// solved again row by row, so that inf and nan spread exactly as in the
+// one-thread sweeps: from its input where the first sweeps or the scans show
+// it (before anything is stored), from the rows' g y where only the second
+// backward sweep, with the carry, goes beyond the range.
 #include "ntk_chunk_f64.h"
 
 #include <algorithm>
@@ -293,10 +295,12 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
   }
   __syncthreads();
   const double xin = t < c.T - 1 ? ex[cur * nt + tid + xs] : 0.0;
-  // whatever is not finite anywhere in the system has reached row 0
-  const bool ok = finite(ex[cur * nt + tid - t * xs]);
+  // what is not finite after these sweeps and scans, anywhere in the system,
+  // has reached row 0
+  bool ok = finite(ex[cur * nt + tid - t * xs]);
 
   // ---- backward again from the carry, results out ----
+  bool over = false;  // a row beyond the range with the carry only: it has reached the chunk's first row
   {
     double* dst = out + base + (long long)r0 * b.es;
     const int k0 = (len - 1) & ~(RB - 1);
@@ -320,9 +324,26 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
 #pragma unroll
       for (int q = 0; q < RB; ++q) v[q] = nx[q];
     }
+    over = ok && len > 0 && !finite(z);
+  }
+  if (__syncthreads_or(over)) {
+    ex[tid] = over ? 1.0 : 0.0;
+    __syncthreads();
+    if (on && ok) {
+      for (int j = 0; j < c.T; ++j) over = over || ex[tid + (j - t) * xs] != 0.0;
+      if (STRIDED && over && t == 0) {  // the rows still hold g y
+        double* dst = out + base;
+        double z = col[slot(c.n - 1)];
+        dst[(long long)(c.n - 1) * b.es] = z;
+        for (int r = c.n - 2; r >= 0; --r) {
+          z = fma(-c.plain.w[r], z, col[slot(r)]);
+          dst[(long long)r * b.es] = z;
+        }
+      }
+      if (!STRIDED && over) ok = false;  // nothing is stored yet
+    }
   }
   if (!STRIDED) {
-    __syncthreads();
     if (on && ok) {
       double* dst = out + base;
 #pragma unroll 4
