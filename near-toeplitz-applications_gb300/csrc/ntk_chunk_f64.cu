@@ -37,7 +37,10 @@
 // solved again row by row, so that inf and nan spread exactly as in the
 // one-thread sweeps: from its input where the first sweeps or the scans show
 // it (before anything is stored), from the rows' g y where only the second
-// backward sweep, with the carry, goes beyond the range.
+// backward sweep, with the carry, goes beyond the range.  A nan in the input
+// reaches every row of a sequential solve, so such systems (masked or diverged
+// fields) are filled instead: 32768 compact lines of 2048 rows, each with a
+// nan, 17500 -> 1330 us (one thread per system: 1110).
 #include "ntk_chunk_f64.h"
 
 #include <algorithm>
@@ -65,11 +68,13 @@ struct ChunkParams {
 
 __device__ __forceinline__ bool finite(double x) { return ((unsigned)__double2hiint(x) & 0x7ff00000u) != 0x7ff00000u; }
 
-// One system row by row from global memory, the forward values parked in out
-// (which may be in: the compact difference keeps its neighbours in registers).
+// One system row by row from global memory, four rows' loads ahead of their
+// dependent FMAs, the forward values parked in out (which may be in: the
+// compact difference keeps its neighbours in registers).
 template <int RHS>
 __device__ __noinline__ void plain_system(const double* in, double* out, long long base, long long es, int n,
                                           long long s, const RhsParams& rp, const TablesF64& t) {
+  constexpr int B = 4;
   const double* a = in + base;
   double* o = out + base;
   double y = 0.0, fm = 0.0, fc = a[0], d0 = fc, dn = 0.0;
@@ -82,32 +87,82 @@ __device__ __noinline__ void plain_system(const double* in, double* out, long lo
     d0 = rp.bnd[s * rp.bnd_ss];
     dn = rp.bnd[s * rp.bnd_ss + (long long)(n - 1) * rp.bnd_es];
   }
-  for (int i = 0; i < n; ++i) {
-    const double* q = a + (long long)i * es;
-    double d;
-    if (RHS == RHS_COMPACT) {
-      const double fn = i < n - 1 ? q[es] : 0.0;
-      d = fn - fm;
-      fm = fc;
-      fc = fn;
-    } else if (RHS == RHS_CROSS) {
-      d = i == 0 || i == n - 1 ? 0.0
-          : rp.center == 0.0   ? -q[-rp.cs] - q[rp.cs]
-                               : fma(rp.top, q[rp.cs], fma(rp.center, q[0], rp.bottom * q[-rp.cs]));
-    } else {
-      d = q[0];
+  for (int i0 = 0; i0 < n; i0 += B) {
+    double d[B], l[B];  // compact: f of the row behind
+#pragma unroll
+    for (int q = 0; q < B; ++q) {
+      const int i = i0 + q;
+      const double* p = a + (long long)i * es;
+      d[q] = 0.0;
+      l[q] = i < n ? t.l[i] : 0.0;
+      if (RHS == RHS_COMPACT) {
+        if (i < n - 1) d[q] = p[es];
+      } else if (RHS == RHS_CROSS) {
+        if (i > 0 && i < n - 1)
+          d[q] = rp.center == 0.0 ? -p[-rp.cs] - p[rp.cs]
+                                  : fma(rp.top, p[rp.cs], fma(rp.center, p[0], rp.bottom * p[-rp.cs]));
+      } else {
+        if (i < n) d[q] = p[0];
+      }
     }
-    if (RHS != RHS_IDENTITY && i == n - 1) d = dn;
-    if (RHS != RHS_IDENTITY && i == 0) d = d0;
-    y = i == 0 ? d : fma(-t.l[i], y, d);
-    o[(long long)i * es] = y;
+#pragma unroll
+    for (int q = 0; q < B; ++q) {
+      const int i = i0 + q;
+      if (i >= n) break;
+      double r = d[q];
+      if (RHS == RHS_COMPACT) {
+        r = d[q] - fm;
+        fm = fc;
+        fc = d[q];
+      }
+      if (RHS != RHS_IDENTITY && i == n - 1) r = dn;
+      if (RHS != RHS_IDENTITY && i == 0) r = d0;
+      y = i == 0 ? r : fma(-l[q], y, r);
+      o[(long long)i * es] = y;
+    }
   }
   double x = t.g[n - 1] * y;
   o[(long long)(n - 1) * es] = x;
-  for (int i = n - 2; i >= 0; --i) {
-    x = fma(-t.w[i], x, t.g[i] * o[(long long)i * es]);
-    o[(long long)i * es] = x;
+  for (int i0 = n - 2; i0 >= 0; i0 -= B) {
+    double e[B], g[B], w[B];
+#pragma unroll
+    for (int q = 0; q < B; ++q) {
+      const int i = max(i0 - q, 0);
+      e[q] = o[(long long)i * es];
+      g[q] = t.g[i];
+      w[q] = t.w[i];
+    }
+#pragma unroll
+    for (int q = 0; q < B; ++q) {
+      if (i0 - q < 0) break;
+      x = fma(-w[q], x, g[q] * e[q]);
+      o[(long long)(i0 - q) * es] = x;
+    }
   }
+}
+
+// Whether rows t, t + T .. of a system show that its sequential solve meets a
+// nan in the forward sweep: a right-hand side that is a nan, or an infinite
+// f_i, 2 <= i <= n - 3, of a compact difference (rows i - 1 and i + 1 then hold
+// infinities of opposite signs, and y_{i+1} is inf - inf whatever the sign of
+// the multipliers).
+template <int RHS>
+__device__ __noinline__ bool meets_nan(const double* a, long long es, int n, int t, int T, long long s,
+                                       const RhsParams& rp) {
+  auto nan = [](double x) { return ((uint64_t)__double_as_longlong(x) & ~(1ull << 63)) > 0x7ffull << 52; };
+  bool seen = false;
+#pragma unroll 1
+  for (int i = t; i < n && !seen; i += T) {
+    const double* q = a + (long long)i * es;
+    if (RHS == RHS_COMPACT)
+      seen = nan(q[0]) || (i > 1 && i < n - 2 && !finite(q[0]));
+    else if (RHS == RHS_CROSS)
+      seen = i == 0 || i == n - 1 ? nan(rp.bnd[s * rp.bnd_ss + (long long)i * rp.bnd_es])
+                                  : nan(q[-rp.cs]) || nan(q[rp.cs]) || (rp.center != 0.0 && nan(q[0]));
+    else
+      seen = nan(q[0]);
+  }
+  return seen;
 }
 
 __device__ __forceinline__ SoftFactor load_factor(const SoftFactor* p) {
@@ -116,7 +171,7 @@ __device__ __forceinline__ SoftFactor load_factor(const SoftFactor* p) {
 }
 
 template <int RHS, bool STRIDED>
-__global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double* out, Batch b,
+__global__ void __launch_bounds__(512, 2) chunk_f64_kernel(const double* in, double* out, Batch b,
                                                         const __grid_constant__ RhsParams rp,
                                                         const __grid_constant__ ChunkParams c) {
   extern __shared__ __align__(16) double smem[];
@@ -326,10 +381,21 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
     }
     over = ok && len > 0 && !finite(z);
   }
-  if (__syncthreads_or(over)) {
+  if (__syncthreads_or(over || (on && !ok))) {
+    // over: chunks beyond the range; where !ok, threads that see a nan
+    if (on && !ok) over = meets_nan<RHS>(in + base, b.es, c.n, t, c.T, sys, rp);
     ex[tid] = over ? 1.0 : 0.0;
     __syncthreads();
-    if (on && ok) {
+    if (on && !ok) {
+      for (int j = 0; j < c.T; ++j) over = over || ex[tid + (j - t) * xs] != 0.0;
+      double* dst = out + base;
+      if (over) {
+        const double x = c.plain.g[0] * __longlong_as_double(0x7ff8ll << 48);
+        for (int r = t; r < c.n; r += c.T) dst[(long long)r * b.es] = x;
+      } else if (t == 0) {
+        plain_system<RHS>(in, out, base, b.es, c.n, sys, rp, c.plain);
+      }
+    } else if (on) {
       for (int j = 0; j < c.T; ++j) over = over || ex[tid + (j - t) * xs] != 0.0;
       if (STRIDED && over && t == 0) {  // the rows still hold g y
         double* dst = out + base;
@@ -340,17 +406,17 @@ __global__ void __launch_bounds__(512) chunk_f64_kernel(const double* in, double
           dst[(long long)r * b.es] = z;
         }
       }
-      if (!STRIDED && over) ok = false;  // nothing is stored yet
+      if (!STRIDED && over) {  // nothing is stored yet
+        ok = false;
+        if (t == 0) plain_system<RHS>(in, out, base, b.es, c.n, sys, rp, c.plain);
+      }
     }
   }
-  if (!STRIDED) {
-    if (on && ok) {
-      double* dst = out + base;
+  if (!STRIDED && on && ok) {
+    double* dst = out + base;
 #pragma unroll 4
-      for (int r = t; r < c.n; r += c.T) dst[r] = col[slot(r)];
-    }
+    for (int r = t; r < c.n; r += c.T) dst[r] = col[slot(r)];
   }
-  if (on && !ok && t == 0) plain_system<RHS>(in, out, base, b.es, c.n, sys, rp, c.plain);
 }
 
 // Pitch of a contiguous system in the tile, in doubles: C + 1, odd, for each
