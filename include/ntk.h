@@ -71,6 +71,13 @@ int ntk_plan_create(ntk_plan** out, int n, long long nrhs, const double coeffs[7
  *                           (default), 1 whole-system shared tile, 2 direct
  *   NTK_TUNE_F64_THREADS    threads per block of the one-thread-per-system
  *                           FP64 kernel: 32, 64, 128 (default)
+ *   NTK_TUNE_F64_CHUNKS     FP64, several threads per system: 0 (default)
+ *                           where a cost rule on the batch expects them to be
+ *                           faster than one thread per system, 1 never, 2
+ *                           wherever the systems fit (n >= 20, a few systems
+ *                           in a CTA's shared memory).  Setting either of the
+ *                           two keys above, which choose among the one-thread
+ *                           kernels, sets this one to 1.
  *   NTK_TUNE_REFINE_W       warps per CTA of the FP32+refine kernel: 4,
  *                           8 (default) or 16 (kernel variants with one
  *                           system per warp, n <= 512 and one sweep; the
@@ -110,7 +117,8 @@ enum ntk_tune_key {
   NTK_TUNE_REFINE_SPW = 4,
   NTK_TUNE_REFINE_KERNEL = 5,
   NTK_TUNE_REFINE_PREFETCH = 6,
-  NTK_TUNE_REFINE_TPS = 7
+  NTK_TUNE_REFINE_TPS = 7,
+  NTK_TUNE_F64_CHUNKS = 8
 };
 int ntk_plan_set_tuning(ntk_plan* plan, int key, int value);
 int ntk_plan_get_tuning(const ntk_plan* plan, int key, int* value);

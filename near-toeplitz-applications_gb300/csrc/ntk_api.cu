@@ -170,8 +170,9 @@ int Plan::run(const double* in, double* out, const Batch& b, RhsParams rp, doubl
     TablesF64 t;
     if ((rc = tables(s, &t))) return rc;
     int S = 0;
-    if (const ChunkF64::Cfg* cfg = chunk_f64_pick(chunk, b, rp.kind, &S))
-      return launch_chunk_f64(chunk, *cfg, S, in, out, b, rp, t, stream);
+    const ChunkF64::Cfg* cfg =
+        tune_f64_chunks == 1 ? nullptr : chunk_f64_pick(chunk, b, rp.kind, &S, tune_f64_chunks == 2);
+    if (cfg) return launch_chunk_f64(chunk, *cfg, S, in, out, b, rp, t, stream);
     return launch_thomas_f64(in, out, n, b, rp, t, tune_f64_threads, stream, tune_f64_x_variant);
   }
   return run_refine(in, out, b, rp, s, stream);
@@ -268,10 +269,16 @@ int ntk_plan_set_tuning(ntk_plan* plan, int key, int value) {
     case NTK_TUNE_F64_X_VARIANT:
       if (value < 0 || value > 2) break;
       plan->tune_f64_x_variant = value;
+      plan->tune_f64_chunks = 1;
       return NTK_OK;
     case NTK_TUNE_F64_THREADS:
       if (value != 32 && value != 64 && value != 128) break;
       plan->tune_f64_threads = value;
+      plan->tune_f64_chunks = 1;
+      return NTK_OK;
+    case NTK_TUNE_F64_CHUNKS:
+      if (value < 0 || value > 2) break;
+      plan->tune_f64_chunks = value;
       return NTK_OK;
     case NTK_TUNE_REFINE_W:
       if (value != 4 && value != 8 && value != 16) break;
@@ -309,6 +316,7 @@ int ntk_plan_get_tuning(const ntk_plan* plan, int key, int* value) {
   switch (key) {
     case NTK_TUNE_F64_X_VARIANT: *value = plan->tune_f64_x_variant; return NTK_OK;
     case NTK_TUNE_F64_THREADS: *value = plan->tune_f64_threads; return NTK_OK;
+    case NTK_TUNE_F64_CHUNKS: *value = plan->tune_f64_chunks; return NTK_OK;
     case NTK_TUNE_REFINE_W: *value = plan->tune_refine_w; return NTK_OK;
     case NTK_TUNE_REFINE_SPW: *value = plan->tune_refine_spw; return NTK_OK;
     case NTK_TUNE_REFINE_KERNEL: *value = plan->tune_refine_kernel; return NTK_OK;

@@ -82,6 +82,7 @@ struct Plan {
   // launch configuration (ntk_plan_set_tuning; chosen by the autotuner)
   int tune_f64_x_variant = 0;  // contiguous FP64 sweeps: 0 tile ring, 1 whole-system tile, 2 direct
   int tune_f64_threads = 128;  // threads per block of the one-thread-per-system FP64 kernel
+  int tune_f64_chunks = 0;     // several threads per system: 0 by the cost rule, 1 never, 2 wherever they fit
   int tune_refine_w = 8;       // warps per CTA of the refinement kernel
   int tune_refine_spw = 1;     // systems per warp (2: strided layouts, 16 rows per lane)
   int tune_refine_kernel = 0;  // n = 512: paired-chunk TMA kernels where they apply (0: automatic, 2: one

@@ -159,9 +159,10 @@ class Plan:
 
     def set_tuning(self, **kw):
         """Set launch parameters (ntk_plan_set_tuning): f64_x_variant,
-        f64_threads, refine_w, refine_spw, refine_kernel, refine_prefetch,
-        refine_tps."""
-        for k, v in kw.items():
+        f64_threads, f64_chunks, refine_w, refine_spw, refine_kernel,
+        refine_prefetch, refine_tps.  f64_chunks is set last: the other two
+        f64 keys set it to 1 (one thread per system)."""
+        for k, v in sorted(kw.items(), key=lambda kv: kv[0] == "f64_chunks"):
             if k not in _lib.TUNE_KEYS:
                 raise ValueError("unknown tuning key %r" % k)
             check(load().ntk_plan_set_tuning(self.handle, _lib.TUNE_KEYS[k], int(v)))

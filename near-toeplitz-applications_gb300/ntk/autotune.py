@@ -9,6 +9,8 @@ cached per (device, kernel family, n, precision, layout):
                  shared tile (threads per system = 1 in both)
   f64_threads    threads per block of the one-thread-per-system FP64 kernel
                  (systems per block for the strided sweeps)
+  f64_chunks     2: several threads per system, offered where a system has
+                 rows for them (the two keys above set it to 1, never)
   refine_w       warps per CTA of the FP32 + refinement kernel (4, 8, 16;
                  threads per system = 32, rows per lane = n / 32 in registers)
   refine_spw     systems per warp (2 stages twice as many adjacent systems
@@ -85,7 +87,8 @@ def cache_key(plan, key):
 
 def candidates(precision, n=None):
     """The configurations searched for a plan of this precision and system
-    length n (threads per system: 64 only offered for 512 < n <= 1024)."""
+    length n (threads per system: 64 only offered for 512 < n <= 1024; several
+    threads per FP64 system from 20 rows on)."""
     out = []
     for space in SPACE.get(precision, [{}]):
         if "refine_kernel" in space:
@@ -95,6 +98,8 @@ def candidates(precision, n=None):
         for name, values in space.items():
             configs = [dict(c, **{name: v}) for c in configs for v in values]
         out += [c for c in configs if c.get("refine_w", 1) * c.get("refine_spw", 1) <= MAX_GROUP]
+    if precision == "fp64" and n is not None and n >= 20:
+        out.append({"f64_chunks": 2})
     return out
 
 
