@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(256, 3)
   const double* t_iu = tk + 2 * LW;
   const double* t_mcu = tk + 3 * LW;
   const double* t_psi = tk + 4 * LW;
-  const uint4* t_siu = reinterpret_cast<const uint4*>(tk - lane + NTAB * LW) + lane;
+  const SoftFactor* t_siu = reinterpret_cast<const SoftFactor*>(tk - lane + NTAB * LW) + lane;
   const double* t_scan = tk + (NTAB + 2) * LW;  // step q: 32 q on, from the other end 32 (5 + q)
   double v[M];
   if (warp < wc) {
@@ -153,19 +153,19 @@ __global__ void __launch_bounds__(256, 3)
   // ---- backward: y / u on the integer pipes, off the dependent chain ----
 #pragma unroll
   for (int k = M - 4; k >= 0; k -= 4) {
-    double y[4];
+    double a[4], y[4];
     bool in_range = true;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const uint4 f4 = __ldg(t_siu + 32 * (k + q));
-      const SoftFactor f{(uint64_t)f4.y << 32 | f4.x, f4.z, f4.w};
-      in_range = in_range && soft_in_range(v[k + q], f);
-      y[q] = soft_product(v[k + q], f);
+      const SoftFactor f = load_factor(t_siu + 32 * (k + q));
+      a[q] = v[k + q];
+      in_range = in_range && soft_in_range(a[q], f, SOFT_SPAN);
+      y[q] = soft_product(a[q], f);
     }
-    if (!in_range) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) y[q] = rare_mul(v[k + q], __ldg(t_iu + 32 * (k + q)));
-    }
+    if (!in_range)
+      rare_rows(
+          a, y, [&](int q) { return __ldg(t_iu + 32 * (k + q)); },
+          [&](int q) { return soft_in_range(a[q], load_factor(t_siu + 32 * (k + q)), SOFT_SPAN); });
 #pragma unroll
     for (int q = 3; q >= 0; --q)
       v[k + q] = k + q == M - 1 ? y[q] : fma(__ldg(t_mcu + 32 * (k + q)), v[(k + q + 1) % M], y[q]);
@@ -250,7 +250,7 @@ bool window_tables(int Lw, int M, const double co[7], double* t) {
   for (int q = 0; q < 5; ++q)
     for (int i = 0; i < Lw; ++i) t[(size_t)q * Lw + (i % M) * 32 + i / M] = (*tabs[q])[i];
   SoftFactor* siu = reinterpret_cast<SoftFactor*>(t + (size_t)5 * Lw);
-  for (int i = 0; i < Lw; ++i) siu[(i % M) * 32 + i / M] = soft_factor(iu[i]);
+  for (int i = 0; i < Lw; ++i) siu[(i % M) * 32 + i / M] = soft_factor(iu[i], SOFT_SPAN);
   // step q of a scan combines lane j with lane j -+ 2^q: the product of the
   // chunks' responses between them, 0 beyond the first (last) lane
   double* up = t + (size_t)7 * Lw;

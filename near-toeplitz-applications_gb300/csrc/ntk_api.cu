@@ -129,7 +129,7 @@ int Plan::g_table(double s, const double** out) {
   for (int i = 0; i < n; ++i) g[i] = s / lu_u[i];
   chunk.g_rows(g.data(), g.data() + rows);
   SoftFactor* sg = reinterpret_cast<SoftFactor*>(g.data() + soft);
-  for (int i = 0; i < n; ++i) sg[i] = soft_factor_untied(g[i]);
+  for (int i = 0; i < n; ++i) sg[i] = soft_factor_untied(g[i], SOFT_SPAN);
   double* d = nullptr;
   int rc = cuda_status(cudaMalloc(&d, sizeof(double) * g.size()), "cudaMalloc(g table)");
   if (rc) return rc;

@@ -233,9 +233,11 @@ __device__ __forceinline__ void f64_window(double* work, double* d, const F64Win
 #pragma unroll
   for (int k = M - 1; k >= 0; --k) {
     f64w_fac(w, pool, r0 + k, l, g, c);
-    const SoftFactor sg = soft_factor(g);
+    const SoftFactor sg = soft_factor(g, SOFT_SPAN);
     double y = soft_product(v[k], sg);
-    if (!soft_in_range(v[k], sg)) y = rare_mul(v[k], g);
+    const bool zero = soft_zero(v[k]) && soft_finite(g);  // padding rows
+    if (zero) y = soft_zero_times(v[k], g);
+    if (!zero && !soft_in_range(v[k], sg, SOFT_SPAN)) y = rare_mul(v[k], g);
     if (k == M - 1) {
       v[k] = y;
       f[k] = -c;

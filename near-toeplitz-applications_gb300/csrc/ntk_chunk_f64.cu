@@ -165,11 +165,6 @@ __device__ __noinline__ bool meets_nan(const double* a, long long es, int n, int
   return seen;
 }
 
-__device__ __forceinline__ SoftFactor load_factor(const SoftFactor* p) {
-  const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
-  return SoftFactor{(uint64_t)q.y << 32 | q.x, q.z, q.w};
-}
-
 template <int RHS, bool STRIDED>
 __global__ void __launch_bounds__(512, 2) chunk_f64_kernel(const double* in, double* out, Batch b,
                                                         const __grid_constant__ RhsParams rp,
@@ -320,13 +315,13 @@ __global__ void __launch_bounds__(512, 2) chunk_f64_kernel(const double* in, dou
       }
 #pragma unroll
       for (int q = 0; q < RB; ++q) {
-        in_range = in_range && (k + q >= len || soft_in_range(v[q], f[q]));
+        in_range = in_range && (k + q >= len || soft_in_range(v[q], f[q], SOFT_SPAN));
         gy[q] = soft_product(v[q], f[q]);
       }
-      if (!in_range) {
-#pragma unroll
-        for (int q = 0; q < RB; ++q) gy[q] = rare_mul(v[q], __ldg(g + k + q));
-      }
+      if (!in_range)
+        rare_rows(
+            v, gy, [&](int q) { return __ldg(g + k + q); },
+            [&](int q) { return k + q >= len || soft_in_range(v[q], load_factor(sg + k + q), SOFT_SPAN); });
 #pragma unroll
       for (int q = RB - 1; q >= 0; --q)
         if (k + q < len) {
@@ -545,7 +540,7 @@ void ChunkF64::g_rows(const double* g, double* out) const {
         const int r = f.rep[j] * f.C + k;
         const size_t at = f.g + (size_t)j * f.C + k;
         plain[at] = r < n ? g[r] : 0.0;
-        sg[at] = soft_factor(plain[at]);
+        sg[at] = soft_factor(plain[at], SOFT_SPAN);
       }
 }
 

@@ -8,7 +8,8 @@
 // rounded to 53 bits, ties to even, i.e. the IEEE product bit for bit.  Ties
 // are common where an operand is short (one product in six for 1.5 or 0.75).
 // Operands outside the range where neither overflow nor underflow can occur
-// (zero, subnormal, inf and nan among them) take the FP64 pipe's product.
+// (subnormal, inf and nan among them) take the FP64 pipe's product; zeros,
+// which are out of that range too, a path of their own (rare_rows).
 // soft_product_untied (41 clocks) rounds half up and serves operands whose
 // product cannot be a tie; the one-thread sweeps, which both pipes bound, take
 // it and leave the others to the FP64 pipe (a 512^3 gradient 2817 -> 2919 us
@@ -34,9 +35,11 @@ namespace ntk {
 
 // A factor prepared for soft_product: mantissa with its leading one in bit
 // 63, and what to add to the other operand's upper word (exponent, and the
-// sign by wrapping).  lim: how many exponents of the other operand, from 64
-// on and in units of its upper word, are served; 0: none (a factor that is
-// zero, not finite or beyond 2^+-60).
+// sign by wrapping).  lim: how many exponents of the other operand, from span
+// + 4 on and in units of its upper word, are served; 0: none (a factor that is
+// zero, not finite or beyond 2^+-span).  The kernels serve factors within
+// 2^+-SOFT_SPAN (coefficients in any units: 1 / dx^2 is beyond 2^60 from dx =
+// 1e-9 on) times operands within 1e+-229.
 struct SoftFactor {
   uint64_t mant;
   uint32_t eadd;
@@ -71,22 +74,24 @@ SOFT_HD double soft_double(uint64_t r) {
 #endif
 }
 
-SOFT_HD SoftFactor soft_factor(double g) {
+constexpr int SOFT_SPAN = 250;
+
+SOFT_HD SoftFactor soft_factor(double g, int span = 60) {
   const uint64_t u = (uint64_t)soft_hi(g) << 32 | soft_lo(g);
   const int e = (int)((u >> 52) & 0x7ff) - 1023;
   SoftFactor f;
   f.mant = (u << 11) | (1ull << 63);
   // the leading one of the rounded mantissa adds one to the exponent field
   f.eadd = ((uint32_t)e << 20) + (uint32_t)(u >> 63 << 31);
-  f.lim = (e >= -60 && e <= 60) ? (1980u - 64u) << 20 : 0u;
+  f.lim = (e >= -span && e <= span) ? (uint32_t)(2036 - 2 * span) << 20 : 0u;
   return f;
 }
 
 // The factor for soft_product_untied: factors of 2 .. 33 significant bits are
 // not served (a product by one of 34 or more bits is no tie unless the
 // operand's lower word is zero, a product by a power of two is exact).
-SOFT_HD SoftFactor soft_factor_untied(double g) {
-  SoftFactor f = soft_factor(g);
+SOFT_HD SoftFactor soft_factor_untied(double g, int span = 60) {
+  SoftFactor f = soft_factor(g, span);
   if ((f.mant & 0x7fffffffull) == 0 && f.mant << 1 != 0) f.lim = 0;
   return f;
 }
@@ -113,8 +118,8 @@ static __device__ __noinline__ double one_sided(double sigma, double f0, double 
 #endif
 
 // whether soft_product serves operand a
-SOFT_HD bool soft_in_range(double a, const SoftFactor& f) {
-  return (soft_hi(a) & 0x7fffffffu) - (64u << 20) < f.lim;
+SOFT_HD bool soft_in_range(double a, const SoftFactor& f, int span = 60) {
+  return (soft_hi(a) & 0x7fffffffu) - ((uint32_t)(span + 4) << 20) < f.lim;
 }
 
 // a times the factor, a in range
@@ -139,7 +144,9 @@ SOFT_HD double soft_product(double a, const SoftFactor& f) {
 }
 
 // whether soft_product_untied is the IEEE product of a and a soft_factor_untied
-SOFT_HD bool soft_untied(double a, const SoftFactor& f) { return soft_in_range(a, f) && soft_lo(a) != 0; }
+SOFT_HD bool soft_untied(double a, const SoftFactor& f, int span = 60) {
+  return soft_in_range(a, f, span) && soft_lo(a) != 0;
+}
 
 SOFT_HD double soft_product_untied(double a, const SoftFactor& f) {
   const uint32_t ah = soft_hi(a), al = soft_lo(a);
@@ -152,5 +159,41 @@ SOFT_HD double soft_product_untied(double a, const SoftFactor& f) {
   }
   return soft_double(((uint64_t)e << 32) + (t >> 11) + ((t >> 10) & 1u));
 }
+
+#ifdef __CUDACC__
+__device__ __forceinline__ SoftFactor load_factor(const SoftFactor* p) {
+  const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+  return SoftFactor{(uint64_t)q.y << 32 | q.x, q.z, q.w};
+}
+#endif
+
+// whether a is +-0, without an FP64 comparison
+SOFT_HD bool soft_zero(double a) { return (soft_hi(a) << 1 | soft_lo(a)) == 0; }
+
+// the zero a times g, g finite
+SOFT_HD double soft_zero_times(double a, double g) {
+  return soft_double((uint64_t)((soft_hi(a) ^ soft_hi(g)) & 0x80000000u) << 32);
+}
+SOFT_HD bool soft_finite(double g) { return (soft_hi(g) & 0x7ff00000u) != 0x7ff00000u; }
+
+#ifdef __CUDACC__
+// y[k] = a[k] g(k) where some of a block's rows are not served(k).  Zeros, of
+// which fields with quiet regions are full, keep off the FP64 pipe here too: a
+// block whose other rows are served keeps their products.
+template <int N, class G, class S>
+__device__ __forceinline__ void rare_rows(const double (&a)[N], double (&y)[N], G g, S served) {
+  bool zeros = true;
+#pragma unroll
+  for (int k = 0; k < N; ++k) zeros = zeros && (served(k) || (soft_zero(a[k]) && soft_finite(g(k))));
+  if (zeros) {
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      if (soft_zero(a[k])) y[k] = soft_zero_times(a[k], g(k));
+  } else {
+#pragma unroll
+    for (int k = 0; k < N; ++k) y[k] = rare_mul(a[k], g(k));
+  }
+}
+#endif
 
 }  // namespace ntk

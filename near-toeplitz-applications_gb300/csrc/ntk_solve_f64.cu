@@ -180,15 +180,14 @@ __device__ __forceinline__ void scaled_rows(const TablesF64& t, int i0, const do
   bool in_range = true;
 #pragma unroll
   for (int k = 0; k < PF; ++k) {
-    const uint4 q = __ldg(reinterpret_cast<const uint4*>(t.sg) + (i0 - k));
-    const SoftFactor f{(uint64_t)q.y << 32 | q.x, q.z, q.w};
-    in_range = in_range && soft_untied(e[k], f);
+    const SoftFactor f = load_factor(t.sg + (i0 - k));
+    in_range = in_range && soft_untied(e[k], f, SOFT_SPAN);
     y[k] = soft_product_untied(e[k], f);
   }
-  if (!in_range) {
-#pragma unroll
-    for (int k = 0; k < PF; ++k) y[k] = rare_mul(e[k], __ldg(t.g + (i0 - k)));
-  }
+  if (!in_range)
+    rare_rows(
+        e, y, [&](int k) { return __ldg(t.g + (i0 - k)); },
+        [&](int k) { return soft_untied(e[k], load_factor(t.sg + (i0 - k)), SOFT_SPAN); });
 }
 
 template <bool VEC>

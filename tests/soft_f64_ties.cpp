@@ -1,7 +1,9 @@
 // soft_product and, where it serves, soft_product_untied
 // (csrc/ntk_soft_f64.cuh) against the host's IEEE product where the exact
 // product may lie halfway between two doubles: short factors times full
-// operands and the reverse.  Prints "checked ties wrong untied wrong".
+// operands and the reverse.  Factors within
+// 2^+-SOFT_SPAN, the kernels' range, with operands of every exponent.  Prints
+// "checked ties wrong untied wrong wide wrong".
 #include <cstdio>
 #include <random>
 
@@ -15,7 +17,7 @@ static double from(uint64_t u) {
 
 int main() {
   std::mt19937_64 r(11);
-  long checked = 0, ties = 0, wrong = 0, untied = 0, wrong2 = 0;
+  long checked = 0, ties = 0, wrong = 0, untied = 0, wrong2 = 0, wide = 0, wrong3 = 0;
   auto check = [&](double a, double g) {
     const ntk::SoftFactor f = ntk::soft_factor(g), f2 = ntk::soft_factor_untied(g);
     if (!ntk::soft_in_range(a, f)) return;
@@ -45,6 +47,17 @@ int main() {
     const uint64_t gb = r() & ~(((uint64_t)1 << (r() % 53)) - 1) & 0x800fffffffffffffull;
     check(a, from(gb | (uint64_t)(1023 - 60 + r() % 121) << 52));
   }
-  std::printf("%ld %ld %ld %ld %ld\n", checked, ties, wrong, untied, wrong2);
+  for (int i = 0; i < 2000000; ++i) {
+    const double a = from(r()), g = from((r() & 0x800fffffffffffffull) | (uint64_t)(1023 - 260 + r() % 521) << 52);
+    const ntk::SoftFactor f = ntk::soft_factor(g, ntk::SOFT_SPAN), f2 = ntk::soft_factor_untied(g, ntk::SOFT_SPAN);
+    if (ntk::soft_in_range(a, f, ntk::SOFT_SPAN)) {
+      ++wide;
+      wrong3 += ntk::soft_product(a, f) != a * g;
+    }
+    if (ntk::soft_untied(a, f2, ntk::SOFT_SPAN)) wrong3 += ntk::soft_product_untied(a, f2) != a * g;
+  }
+  for (double g : {1e76, -1e-76, 0.0})  // beyond the span
+    wrong3 += ntk::soft_in_range(1.0, ntk::soft_factor(g, ntk::SOFT_SPAN), ntk::SOFT_SPAN);
+  std::printf("%ld %ld %ld %ld %ld %ld %ld\n", checked, ties, wrong, untied, wrong2, wide, wrong3);
   return 0;
 }

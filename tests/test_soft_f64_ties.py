@@ -18,9 +18,10 @@ def test_ties_round_to_even(tmp_path):
     subprocess.run(["g++", "-O2", "-std=c++17", "-I", os.path.join(PKG_DIR, "csrc"), "-I", cuda, "-o", str(exe),
                     os.path.join(ROOT, "tests", "soft_f64_ties.cpp")], check=True)
     res = subprocess.run([str(exe)], stdout=subprocess.PIPE, check=True).stdout
-    checked, ties, wrong, untied, wrong_untied = map(int, res.split())
+    checked, ties, wrong, untied, wrong_untied, wide, wrong_wide = map(int, res.split())
     assert checked > 4000000 and ties > 50000 and untied > 100000
     assert wrong == 0 and wrong_untied == 0
+    assert wide > 500000 and wrong_wide == 0
 
 
 # 3 systems: several threads a system; 300000: one thread a system
