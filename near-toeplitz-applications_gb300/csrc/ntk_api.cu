@@ -107,16 +107,17 @@ int Plan::init(int n_, long long nrhs_, const double co[7], int prec, int sweeps
 
 Plan::~Plan() {
   if (d_lw) cudaFree(d_lw);
-  for (auto& kv : g_by_scale) cudaFree(kv.second);
+  for (auto& kv : g_by_scale) cudaFree(kv.second.d);
   release_refine();
 }
 
 // g_i = s / u_i for the requested scale, uploaded once per distinct s.
-int Plan::g_table(double s, const double** out) {
+int Plan::g_table(double s, const double** out, bool* soft_served) {
   std::lock_guard<std::mutex> lk(mu);
   auto it = g_by_scale.find(s);
   if (it != g_by_scale.end()) {
-    *out = it->second;
+    *out = it->second.d;
+    if (soft_served) *soft_served = it->second.soft;
     return NTK_OK;
   }
   if (g_by_scale.size() >= 16) {
@@ -129,7 +130,11 @@ int Plan::g_table(double s, const double** out) {
   for (int i = 0; i < n; ++i) g[i] = s / lu_u[i];
   chunk.g_rows(g.data(), g.data() + rows);
   SoftFactor* sg = reinterpret_cast<SoftFactor*>(g.data() + soft);
-  for (int i = 0; i < n; ++i) sg[i] = soft_factor_untied(g[i], SOFT_SPAN);
+  int refused = 0;
+  for (int i = 0; i < n; ++i) {
+    sg[i] = soft_factor_untied(g[i], SOFT_SPAN);
+    refused += sg[i].lim == 0;
+  }
   double* d = nullptr;
   int rc = cuda_status(cudaMalloc(&d, sizeof(double) * g.size()), "cudaMalloc(g table)");
   if (rc) return rc;
@@ -138,16 +143,22 @@ int Plan::g_table(double s, const double** out) {
     cudaFree(d);
     return rc;
   }
-  g_by_scale[s] = d;
+  // a row that is refused costs its block the integer and the FP64 products:
+  // a matrix of short factors (few distinct rows, such as diagonal ones) keeps
+  // the FP64 products
+  const GTable e{d, refused <= n / 16};
+  g_by_scale[s] = e;
   *out = d;
+  if (soft_served) *soft_served = e.soft;
   return NTK_OK;
 }
 
 int Plan::tables(double s, TablesF64* t) {
   t->l = d_lw;
   t->w = d_lw + n;
-  const int rc = g_table(s, &t->g);
-  if (!rc)
+  bool soft = false;
+  const int rc = g_table(s, &t->g, &soft);
+  if (!rc && soft)
     t->sg = reinterpret_cast<const SoftFactor*>(t->g + chunk.g_offset(n) + ((chunk.g_elems() + 1) & ~(size_t)1));
   return rc;
 }

@@ -109,7 +109,7 @@ struct TablesF64 {
   const double* l = nullptr;  // l_i = a_i / u_{i-1}
   const double* g = nullptr;  // g_i = s / u_i
   const double* w = nullptr;  // w_i = c_i / u_i
-  const SoftFactor* sg = nullptr;  // g_i prepared for soft_product_untied (Plan::tables)
+  const SoftFactor* sg = nullptr;  // g_i prepared for soft_product_untied, or null (Plan::tables)
 };
 
 void set_error(const char* fmt, ...);

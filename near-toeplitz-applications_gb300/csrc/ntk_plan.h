@@ -71,7 +71,11 @@ struct Plan {
   std::vector<double> lu_l, lu_u;   // host LU factors (FP64)
   double* d_lw = nullptr;           // device: l[n], w[n]
   ChunkF64 chunk;                   // NTK_FP64 with few systems: T threads per system
-  std::map<double, double*> g_by_scale;  // device g tables (g = s/u) per RHS scale
+  struct GTable {
+    double* d = nullptr;
+    bool soft = false;  // nearly all factors are served by soft_product_untied
+  };
+  std::map<double, GTable> g_by_scale;  // device g tables (g = s/u) per RHS scale
   RefineState* refine = nullptr;
   LongRefine* long_refine = nullptr;  // FP32 / FP32+refine windows for n > 1024
   SpikeSolver* spike = nullptr;       // n > 1024 where the windows' halos do not decay: exact partitions
@@ -93,7 +97,7 @@ struct Plan {
 
   int init(int n, long long nrhs, const double co[7], int precision, int sweeps);
   ~Plan();
-  int g_table(double s, const double** out);
+  int g_table(double s, const double** out, bool* soft = nullptr);
   int tables(double s, TablesF64* t);  // l, w and the g table of scale s
   int check_device() const;
   int run(const double* in, double* out, const Batch& b, RhsParams rp, double s, cudaStream_t stream);

@@ -14,9 +14,10 @@
 //   forward   eta_i = D_i - l_i * eta_{i-1}          (1 DFMA; +1 DADD for the
 //                                                      compact RHS difference)
 //   backward  x_i  = g_i * eta_i - w_i * x_{i+1}     (1 DFMA; g_i eta_i off the
-//                                                      chain, on the integer pipes)
-// i.e. 2 (in-place solve) or 3 (fused compact derivative) FP64 instructions
-// per unknown, against ~10 plus two FP64 divisions per unknown in the
+//                                                      chain: 1 DMUL, or with many
+//                                                      systems the integer pipes)
+// i.e. 2 or 3 (in-place solve), 3 or 4 (fused compact derivative) FP64
+// instructions per unknown, against ~10 plus two FP64 divisions per unknown in the
 // reference's cyclic reduction.  Nothing else may touch the FP64 pipe in the
 // row loops: a condition on the row (first, last) around FP64 work becomes
 // predicated instructions there, which hold the pipe like executed ones, so
@@ -172,11 +173,17 @@ __device__ __forceinline__ double forward_compact(const double* src, double* dst
 
 // ----------------------------------------------------------------------------
 // backward sweep: x_i = g_i eta_i - w_i x_{i+1}, eta read back from dst.
-// g eta runs on the integer pipes (ntk_soft_f64.cuh), PF rows at a time with
-// one range check, which leaves one FP64 instruction a row.
+// With SOFT g eta runs on the integer pipes (ntk_soft_f64.cuh), PF rows at a
+// time with one range check, which leaves one FP64 instruction a row.
 // ----------------------------------------------------------------------------
 // y[k] = g_{i0 - k} e[k], k < PF
+template <bool SOFT>
 __device__ __forceinline__ void scaled_rows(const TablesF64& t, int i0, const double (&e)[PF], double (&y)[PF]) {
+  if (!SOFT) {
+#pragma unroll
+    for (int k = 0; k < PF; ++k) y[k] = __ldg(t.g + (i0 - k)) * e[k];
+    return;
+  }
   bool in_range = true;
 #pragma unroll
   for (int k = 0; k < PF; ++k) {
@@ -190,7 +197,7 @@ __device__ __forceinline__ void scaled_rows(const TablesF64& t, int i0, const do
         [&](int k) { return soft_untied(e[k], load_factor(t.sg + (i0 - k)), SOFT_SPAN); });
 }
 
-template <bool VEC>
+template <bool SOFT>
 __device__ __forceinline__ void backward(double* dst, long long es, int n, double eta_last, const TablesF64& t) {
   double x = __ldg(t.g + (n - 1)) * eta_last;
   dst[(long long)(n - 1) * es] = x;
@@ -203,8 +210,18 @@ __device__ __forceinline__ void backward(double* dst, long long es, int n, doubl
   }
   int i = n - 2;  // ring[k]: row i - k
   for (; i >= PF - 1; i -= PF) {
+    if (!SOFT) {  // each row's successor in the ring on its way before the row is used
+#pragma unroll
+      for (int k = 0; k < PF; ++k) {
+        const double e = ring[k];
+        if (i - k - PF >= 0) ring[k] = dst[(long long)(i - k - PF) * es];
+        x = fma(-__ldg(t.w + (i - k)), x, __ldg(t.g + (i - k)) * e);
+        dst[(long long)(i - k) * es] = x;
+      }
+      continue;
+    }
     double y[PF];
-    scaled_rows(t, i, ring, y);
+    scaled_rows<SOFT>(t, i, ring, y);
 #pragma unroll
     for (int k = 0; k < PF; ++k)
       if (i - k - PF >= 0) ring[k] = dst[(long long)(i - k - PF) * es];
@@ -222,7 +239,7 @@ __device__ __forceinline__ void backward(double* dst, long long es, int n, doubl
     }
 }
 
-template <int RHS, bool VEC>
+template <int RHS, bool VEC, bool SOFT>
 __global__ void __launch_bounds__(128) thomas_f64_kernel(const double* in, double* out, int n, Batch b,
                                                          RhsParams rp, TablesF64 t) {
   const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -243,7 +260,7 @@ __global__ void __launch_bounds__(128) thomas_f64_kernel(const double* in, doubl
     eta = fma(-__ldg(t.l + (n - 1)), eta, rp.sigmaN * ((-5.0 * fl2 + 4.0 * fl1) + fl0));
     dst[(long long)(n - 1) * b.es] = eta;
   }
-  backward<VEC>(dst, b.es, n, eta, t);
+  backward<SOFT>(dst, b.es, n, eta, t);
 }
 
 // ----------------------------------------------------------------------------
@@ -463,7 +480,7 @@ __device__ __forceinline__ void xtile_store(const double* tile, double* base0, l
   }
 }
 
-template <int RHS>
+template <int RHS, bool SOFT>
 __global__ void __launch_bounds__(32 * XWARPS) thomas_f64_xpose_kernel(const double* in, double* out, int n, Batch b,
                                                                        RhsParams rp, TablesF64 t) {
   extern __shared__ __align__(16) double xsm[];
@@ -565,7 +582,7 @@ __global__ void __launch_bounds__(32 * XWARPS) thomas_f64_xpose_kernel(const dou
       double e[PF], y[PF];
 #pragma unroll
       for (int q = 0; q < PF; ++q) e[q] = cur[(k - q) * XP + lane];
-      scaled_rows(t, row0 + k, e, y);
+      scaled_rows<SOFT>(t, row0 + k, e, y);
 #pragma unroll
       for (int q = 0; q < PF; ++q) {
         x = fma(-__ldg(t.w + (row0 + k - q)), x, y[q]);
@@ -601,18 +618,24 @@ int launch_thomas_f64(const double* in, double* out, int n, const Batch& b, cons
   // contiguous systems, 32 per warp equally spaced: transposing tile ring
   const bool xlike = (b.es == 1) && (b.ni >= b.nsys || b.ni % 32 == 0) && (rp.kind == RHS_IDENTITY || n >= 4) &&
                      (rp.kind == RHS_IDENTITY || rp.kind == RHS_COMPACT);
+  // g eta on the integer pipes where the FP64 pipe bounds the sweeps.  Below
+  // that many warps a sub-partition the rows' latency does, to which the
+  // integer product adds more than the FP64 one.  Strided solves of 512 rows,
+  // us, FP64 product : integer, of a field of zeros: 32768 systems (2 warps)
+  // 191 : 167, 190 : 239; 65536 (4) 244 : 202, 243 : 276; 131072 (7) 433 :
+  // 328, 434 : 406; compact 8192 (1) 107 : 112, 107 : 171; 131072 542 : 450,
+  // 541 : 524.  Contiguous ones (tiles): 50000 (3) 242 : 272, 243 : 310;
+  // 131072 559 : 566, 555 : 684; of 64 rows 75 : 67, 75 : 83.
+  const long long warps = (b.nsys + 31) / 32, load = (warps + 4 * 152 - 1) / (4 * 152);
+  const bool soft = t.sg && load >= (xlike && x_variant == 0 ? 6 : 5);
   if (xlike && x_variant == 0) {
     const size_t xs = (size_t)XWARPS * XRING * XT * XP * sizeof(double);
     const long long xblocks = (b.nsys + 32 * XWARPS - 1) / (32 * XWARPS);
-    if (rp.kind == RHS_IDENTITY) {
-      auto k = thomas_f64_xpose_kernel<RHS_IDENTITY>;
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xs);
-      k<<<(unsigned)xblocks, 32 * XWARPS, xs, stream>>>(in, out, n, b, rp, t);
-    } else {
-      auto k = thomas_f64_xpose_kernel<RHS_COMPACT>;
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xs);
-      k<<<(unsigned)xblocks, 32 * XWARPS, xs, stream>>>(in, out, n, b, rp, t);
-    }
+    auto k = rp.kind == RHS_IDENTITY
+                 ? (soft ? thomas_f64_xpose_kernel<RHS_IDENTITY, true> : thomas_f64_xpose_kernel<RHS_IDENTITY, false>)
+                 : (soft ? thomas_f64_xpose_kernel<RHS_COMPACT, true> : thomas_f64_xpose_kernel<RHS_COMPACT, false>);
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)xs);
+    k<<<(unsigned)xblocks, 32 * XWARPS, xs, stream>>>(in, out, n, b, rp, t);
     return cuda_status(cudaGetLastError(), "thomas_f64_xpose_kernel");
   }
   // contiguous systems that fit a 32-system tile in shared memory: staged kernel
@@ -632,15 +655,13 @@ int launch_thomas_f64(const double* in, double* out, int n, const Batch& b, cons
     return cuda_status(cudaGetLastError(), "thomas_f64_staged_kernel");
   }
   if (rp.kind == RHS_IDENTITY) {
-    if (vec)
-      thomas_f64_kernel<RHS_IDENTITY, true><<<grid, block, 0, stream>>>(in, out, n, b, rp, t);
-    else
-      thomas_f64_kernel<RHS_IDENTITY, false><<<grid, block, 0, stream>>>(in, out, n, b, rp, t);
+    auto k = vec ? (soft ? thomas_f64_kernel<RHS_IDENTITY, true, true> : thomas_f64_kernel<RHS_IDENTITY, true, false>)
+                 : (soft ? thomas_f64_kernel<RHS_IDENTITY, false, true> : thomas_f64_kernel<RHS_IDENTITY, false, false>);
+    k<<<grid, block, 0, stream>>>(in, out, n, b, rp, t);
   } else if (rp.kind == RHS_COMPACT) {
-    if (vec)
-      thomas_f64_kernel<RHS_COMPACT, true><<<grid, block, 0, stream>>>(in, out, n, b, rp, t);
-    else
-      thomas_f64_kernel<RHS_COMPACT, false><<<grid, block, 0, stream>>>(in, out, n, b, rp, t);
+    auto k = vec ? (soft ? thomas_f64_kernel<RHS_COMPACT, true, true> : thomas_f64_kernel<RHS_COMPACT, true, false>)
+                 : (soft ? thomas_f64_kernel<RHS_COMPACT, false, true> : thomas_f64_kernel<RHS_COMPACT, false, false>);
+    k<<<grid, block, 0, stream>>>(in, out, n, b, rp, t);
   } else {
     set_error("unsupported RHS kind %d for the FP64 solve", rp.kind);
     return NTK_ERR_INVALID;
