@@ -96,10 +96,13 @@ int ntk_plan_create(ntk_plan** out, int n, long long nrhs, const double coeffs[7
  *                           (default) picks 3 for NTK_FP32 and 2 for
  *                           NTK_FP32_REFINE (faster on GB300); 1 the
  *                           chunked kernel above.  Other n >= 96 and
- *                           layouts, one sweep: 1 the chunked kernel, else
- *                           paired chunks of any number where the factors
- *                           decay within 16 rows and the batch fills the
- *                           GPU.  With 0, 2 or 3,
+ *                           layouts, one sweep, where both LU multipliers of
+ *                           the interior are at most 0.324 (16 rows decay by
+ *                           2^26; backward Euler up to r = 0.71): 1 the
+ *                           chunked kernels, 2 or 3 paired chunks of any
+ *                           number, 0 these where a rule on the batch expects
+ *                           them to be faster; NTK_TUNE_REFINE_TPS = 64 keeps
+ *                           the chunked kernels.  For n = 512, with 0, 2 or 3,
  *                           NTK_TUNE_REFINE_W sets the systems per CTA of
  *                           contiguous layouts (4, 8 or 16).
  *   NTK_TUNE_REFINE_PREFETCH  the one-group strided kernel: a CTA prefetches

@@ -34,8 +34,8 @@
 // Measured against the chunked kernels, us: derivatives of a 240 x 385 x 700
 // field along x (700 rows) 814 -> 304, y (385) 448 -> 341, z (240) 439 -> 277;
 // 16384 systems of 2048 rows in place 281 -> 185, 65536 of 100 rows 60 -> 37,
-// 2600 of 300 rows 12.6 -> 10.5.  Below one group per SM the chunked kernels
-// keep the batch.
+// 2600 of 300 rows 12.6 -> 10.5.  Smaller batches stay with the chunked
+// kernels (r2n_serves).
 #include "ntk_r2n.h"
 
 #include <algorithm>
@@ -717,7 +717,29 @@ int r2n_create(R2N** out, const Plan& p) {
   return NTK_OK;
 }
 
-bool r2n_serves(const R2N* r, const double* in, const double* out, const Batch& b, const RhsParams& rp) {
+namespace {
+
+// Whether tensor maps address the strided systems of a batch.
+bool maps_apply(const double* in, const Batch& b, long long planes) {
+  return r2::aligned16(in) && b.es % 2 == 0 && (planes == 1 || b.os % 2 == 0);
+}
+
+}  // namespace
+
+// Which batches take this kernel rather than the chunked ones (one warp a
+// system), by the threads it gives an SM: a CTA's time is mostly latency, and
+// staging without tensor maps (8-byte copies) adds to it, so it takes several
+// a SM to win.  Measured, us, this kernel : the chunked ones, with threads an
+// SM: contiguous 2432 systems of 128 rows (128) 5.7 : 4.0, 8192 (431) 8.3 :
+// 8.5, 4868 of 256 (513) 8.6 : 9.2, 8191 of 97, odd (377) 10.4 : 9.1, 12001
+// (553) 12.0 : 12.5; strided with tensor maps 2560 of 256 (269) 7.4 : 7.1, 4868
+// (514) 9.2 : 10.0; without 4867 of 500 (1027) 20.2 : 18.0, 8191 (1725) 27.6 :
+// 26.7, 12001 of 385 (2372) 31.8 : 34.8; windows in place, in order, strided
+// 2432 of 1024 (256) 24.4 : 18.5, 4868 (514) 42.2 : 40.7, 6400 (674) 42.9 :
+// 50.1; contiguous 2437 of 2048 (401) 45.7 : 43.8, 3600 of 1024 (568) 23.5 :
+// 25.6.
+bool r2n_serves(const R2N* r, const double* in, const double* out, const Batch& b, const RhsParams& rp,
+                bool always) {
   if (!r || b.nsys < 1 || (rp.kind != RHS_IDENTITY && rp.kind != RHS_COMPACT)) return false;
   if (b.nsys > b.ni && b.nsys % b.ni != 0) return false;
   const long long planes = b.nsys > b.ni ? b.nsys / b.ni : 1, ni = b.nsys / planes;
@@ -733,8 +755,13 @@ bool r2n_serves(const R2N* r, const double* in, const double* out, const Batch& 
   const long long extent = (planes - 1) * b.os + plane;
   if (in != out && in < out + extent && out < in + extent) return false;
   // windows in place: all of a system's windows in one CTA
-  if (in == out && y.P > 1) return rp.kind == RHS_IDENTITY && groups >= r->sms;
-  return groups * y.P >= r->sms;
+  const bool seq = in == out && y.P > 1;
+  if (seq && rp.kind != RHS_IDENTITY) return false;
+  if (always) return true;
+  const bool contig = b.es == 1;
+  int least = seq ? (contig ? 448 : 640) : 384;
+  if (!contig && !maps_apply(in, b, planes)) least = r->n <= 512 ? 1280 : seq ? 1024 : 768;
+  return (seq ? groups : groups * y.P) * (sg * y.nc) >= (long long)least * r->sms;
 }
 
 namespace {
@@ -785,7 +812,7 @@ int r2n_run(R2N* r, const double* in, double* out, const Batch& b, const RhsPara
   const long long groups = (long long)g.gpp * planes;
   CUtensorMap map;
   std::memset(&map, 0, sizeof(map));
-  if (!contig && r2::aligned16(in) && b.es % 2 == 0 && (planes == 1 || b.os % 2 == 0)) {
+  if (!contig && maps_apply(in, b, planes)) {
     g.boxr = y.Wr > 256 ? y.Wr / 2 : y.Wr;
     const cuuint64_t dims[4] = {(cuuint64_t)ni, (cuuint64_t)r->n, (cuuint64_t)planes, 1};
     const long long ps = planes > 1 ? b.os : (long long)b.es * r->n;

@@ -15,7 +15,8 @@ void r2n_destroy(R2N* r);
 void r2n_status_words(const R2N* r, std::vector<unsigned*>& out);
 
 // Whether r2n_run serves this batch (one refinement sweep) and is the faster.
-bool r2n_serves(const R2N* r, const double* in, const double* out, const Batch& b, const RhsParams& rp);
+bool r2n_serves(const R2N* r, const double* in, const double* out, const Batch& b, const RhsParams& rp,
+                bool always = false);
 int r2n_run(R2N* r, const double* in, double* out, const Batch& b, const RhsParams& rp, double s, int prefetch,
             cudaStream_t st);
 

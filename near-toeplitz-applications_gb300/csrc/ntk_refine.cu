@@ -229,7 +229,8 @@ int Plan::run_refine(const double* in, double* out, const Batch& b, const RhsPar
                      cudaStream_t stream) {
   // every length but the 512-row kernels' own
   const bool own_512 = refine && refine->r2_ok && r2::layout_ok(in, out, b);
-  if (!own_512 && tune_refine_kernel != 1 && tune_refine_tps != 64 && r2n_serves(r2n, in, out, b, rp))
+  if (!own_512 && tune_refine_kernel != 1 && tune_refine_tps != 64 &&
+      r2n_serves(r2n, in, out, b, rp, tune_refine_kernel != 0))
     return r2n_run(r2n, in, out, b, rp, s, tune_refine_prefetch, stream);
   if (spike) {
     if (rp.kind != RHS_IDENTITY || s != 1.0) {
