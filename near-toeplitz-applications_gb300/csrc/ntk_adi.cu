@@ -208,6 +208,7 @@ int ntk_adi_create(ntk_adi** out, int N, double dx, double dt, int precision) {
   a->bottom = -1. / (dx * dx);
   a->top = -1. / (dx * dx);
   a->center = 2 * (-1. / dt + 1. / (dx * dx));
+  a->plan.factors_only = true;
   int rc = a->plan.init(N, N - 2, co, NTK_FP64, 1);
   if (rc == NTK_OK) {
     std::vector<double> w(N);

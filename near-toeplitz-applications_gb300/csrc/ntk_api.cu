@@ -91,18 +91,22 @@ int Plan::init(int n_, long long nrhs_, const double co[7], int prec, int sweeps
     set_error("matrix has a zero or non-finite pivot (LU breakdown)");
     return NTK_ERR_INVALID;
   }
-  // l and w are independent of the RHS scale
+  // l and w are independent of the RHS scale; the chunk tables lie behind them
+  // (one allocation and one copy: they are most of a plan's creation)
   std::vector<double> host(2 * (size_t)n);
   for (int i = 0; i < n; ++i) {
     host[i] = lu_l[i];
     host[n + i] = (i < n - 1 ? mat.c(i) : 0.0) / lu_u[i];
   }
-  int rc = cuda_status(cudaMalloc(&d_lw, sizeof(double) * 2 * (size_t)n), "cudaMalloc(factor tables)");
+  if (precision == NTK_FP64 && !factors_only) {
+    const std::vector<double> tab = chunk.init(n, lu_l.data(), lu_u.data(), host.data() + n);
+    host.insert(host.end(), tab.begin(), tab.end());
+  }
+  int rc = cuda_status(cudaMalloc(&d_lw, sizeof(double) * host.size()), "cudaMalloc(factor tables)");
   if (rc) return rc;
-  rc = cuda_status(cudaMemcpy(d_lw, host.data(), sizeof(double) * 2 * (size_t)n, cudaMemcpyHostToDevice),
-                   "cudaMemcpy(factor tables)");
-  if (rc || precision != NTK_FP64) return rc;
-  return chunk.init(n, lu_l.data(), lu_u.data(), host.data() + n);
+  chunk.d_tab = d_lw + 2 * (size_t)n;
+  return cuda_status(cudaMemcpy(d_lw, host.data(), sizeof(double) * host.size(), cudaMemcpyHostToDevice),
+                     "cudaMemcpy(factor tables)");
 }
 
 Plan::~Plan() {

@@ -446,11 +446,7 @@ int launch_one(const double* in, double* out, const Batch& b, const RhsParams& r
 
 }  // namespace
 
-ChunkF64::~ChunkF64() {
-  if (d_tab) cudaFree(d_tab);
-}
-
-int ChunkF64::init(int n_, const double* l, const double* u, const double* w) {
+std::vector<double> ChunkF64::init(int n_, const double* l, const double* u, const double* w) {
   n = n_;
   std::vector<double> tab;
   for (int T = 4; T <= MAXT; T *= 2) {
@@ -517,12 +513,7 @@ int ChunkF64::init(int n_, const double* l, const double* u, const double* w) {
     g_count += (size_t)f.ncls * f.C;
     cfgs.push_back(f);
   }
-  if (cfgs.empty()) return NTK_OK;
-  int rc = cuda_status(cudaMalloc(&d_tab, tab.size() * sizeof(double)), "cudaMalloc(chunk tables)");
-  if (!rc)
-    rc = cuda_status(cudaMemcpy(d_tab, tab.data(), tab.size() * sizeof(double), cudaMemcpyHostToDevice),
-                     "cudaMemcpy(chunk tables)");
-  return rc;
+  return tab;
 }
 
 bool ChunkF64::serves_both_layouts() const {

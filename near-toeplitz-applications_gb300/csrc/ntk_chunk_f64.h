@@ -22,13 +22,12 @@ struct ChunkF64 {
   };
   int n = 0;
   std::vector<Cfg> cfgs;
-  double* d_tab = nullptr;
+  const double* d_tab = nullptr;  // the plan's copy of init's tables
   size_t g_count = 0;      // rows of g of all configurations
 
-  ~ChunkF64();
-  // l, u: the matrix's LU factors, w = c / u.  Leaves cfgs empty where no
-  // thread count applies; fails only where an allocation or a copy does.
-  int init(int n, const double* l, const double* u, const double* w);
+  // l, u: the matrix's LU factors, w = c / u.  Returns the tables for the
+  // device; leaves cfgs empty where no thread count applies.
+  std::vector<double> init(int n, const double* l, const double* u, const double* w);
   // whether some configuration fits contiguous and some strided systems
   bool serves_both_layouts() const;
   // A g table holds g[n] and, from g_offset(n) on, the rows of g in chunk

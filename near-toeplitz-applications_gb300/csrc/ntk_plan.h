@@ -69,7 +69,7 @@ struct Plan {
   int sweeps = 1;
   int device = -1;
   std::vector<double> lu_l, lu_u;   // host LU factors (FP64)
-  double* d_lw = nullptr;           // device: l[n], w[n]
+  double* d_lw = nullptr;           // device: l[n], w[n], chunk tables
   ChunkF64 chunk;                   // NTK_FP64 with few systems: T threads per system
   struct GTable {
     double* d = nullptr;
@@ -79,6 +79,7 @@ struct Plan {
   RefineState* refine = nullptr;
   LongRefine* long_refine = nullptr;  // FP32 / FP32+refine windows for n > 1024
   SpikeSolver* spike = nullptr;       // n > 1024 where the windows' halos do not decay: exact partitions
+  bool factors_only = false;          // a matrix whose LU factors are wanted, no solves by this plan itself
   bool window_tables = false;         // a window matrix of another plan: tables only, no batches of its own
   R2N* r2n = nullptr;                 // one sweep, any n: paired chunks (null where they do not apply)
   LongRefine* long_alt = nullptr;     // 512 < n <= 1024: two-window solve (64 threads per system)
