@@ -3,7 +3,7 @@
 The reference fixes its launch configuration in jinja2 templates
 (neato.py:160-163: one thread per even row, one block per system).  Here the
 launch parameters of a plan are searched by timing on the current GPU and
-cached per (device, kernel family, n, precision, layout):
+cached per (device, kernel set, n, precision, layout):
 
   f64_x_variant  contiguous FP64 sweeps: transposing tile ring / whole-system
                  shared tile (threads per system = 1 in both)
@@ -19,7 +19,9 @@ cached per (device, kernel family, n, precision, layout):
                  thread, two 8-row halves per packed FP32x2 instruction;
                  refine_w = systems per CTA of contiguous layouts) with one
                  strided group per CTA (2) or persistent strided CTAs (3);
-                 1 the chunked kernel (refine_w, refine_spw as above)
+                 1 the chunked kernel (refine_w, refine_spw as above).
+                 Other n: 2 and 3 the paired chunks of any number, which
+                 read refine_prefetch only
   refine_prefetch  one-group strided CTAs: L2 prefetch of the tile needed
                  p / 2 waves later (p = 1, 2, 3 searched; 0 and 4, no
                  prefetch and two waves, measured slower on every axis)
@@ -49,6 +51,9 @@ SPACE = {
                     {"refine_kernel": [3], "refine_w": [4, 8, 16]},
                     {"refine_kernel": [1], "refine_w": [4, 8, 16], "refine_spw": [1, 2]}],
 }
+# Raised with every change of the kernels or of what a parameter selects: a
+# result cached for other kernels is searched anew.
+KERNEL_SET = 2
 # a refinement CTA stages at most 16 systems (refine_w * refine_spw)
 MAX_GROUP = 16
 
@@ -82,7 +87,7 @@ def device_name():
 
 
 def cache_key(plan, key):
-    return "|".join([device_name(), str(plan.n), str(plan.precision), str(key)])
+    return "|".join([device_name(), "k%d" % KERNEL_SET, str(plan.n), str(plan.precision), str(key)])
 
 
 def candidates(precision, n=None):
