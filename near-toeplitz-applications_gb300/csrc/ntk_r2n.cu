@@ -45,6 +45,7 @@
 #include "ntk_device.cuh"
 #include "ntk_r2_host.h"
 #include "ntk_r2_tma.cuh"
+#include "ntk_r2n_windows.h"
 
 namespace ntk {
 namespace r2n {
@@ -55,7 +56,6 @@ using namespace r2;
 // fills an SM's threads better (384 rows: 5 CTAs of 192 threads, not 2 of 384)
 template <bool CONTIG>
 constexpr int group_size = CONTIG ? 8 : 16;
-constexpr int MAX_NC = 32;    // chunks of a window
 // exchange values, [chunk][value][system] floats: a neighbour's are a constant
 // distance away, and the chunks of a warp use different banks
 enum { X_E1 = 0, X_S1, X_A0, X_B0, X_B7, X_E2, X_S2, X_COUNT };
@@ -526,8 +526,8 @@ __global__ void __launch_bounds__(512, 2)
 }  // namespace r2n
 
 struct R2N {
-  struct Layout {
-    int H = 0, P = 1, Wr = 0, nc = 0;
+  struct Layout : r2n::Windows {
+    int nc = 0;  // chunks of a window
   };
   int n = 0;
   Layout lay[2];  // strided, contiguous
@@ -610,31 +610,13 @@ int r2n_create(R2N** out, const Plan& p) {
   int H = 0;
   for (double q = 1.0; q > std::ldexp(1.0, -56); q *= mult) ++H;
   H = (H + 3) & ~1;  // even: window starts stay 16-byte aligned
-  // windows: the fewest rows solved for the share of the 1024 threads (64
-  // registers each) that whole CTAs can fill; several small CTAs overlap their
-  // phases better than two large ones
   for (int lay = 0; lay < 2; ++lay) {
-    const int sg = lay ? group_size<true> : group_size<false>;
     R2N::Layout& y = r->lay[lay];
-    double best = 0.0;
-    for (int P = 1; P <= 4096; ++P) {
-      const int Wr = (int)(((long long)n + 2LL * H * (P - 1) + 16 * P - 1) / (16 * P)) * 16;
-      if (P > 1 && Wr < 4 * H + 64) break;  // halos would be half of the work
-      if (Wr > 16 * MAX_NC) continue;
-      const int threads = Wr / 16 * sg, ctas = std::min(1024 / threads, 32);
-      const double cost = (double)P * Wr / (ctas * threads * (1.0 - 0.1 / ctas));
-      if (best == 0.0 || cost < best) {
-        best = cost;
-        y.P = P;
-        y.Wr = Wr;
-      }
-      if (P > 1 && P * (long long)(512 - 2 * H) > 4LL * n) break;
-    }
-    if (best == 0.0) {
+    static_cast<Windows&>(y) = choose_windows(n, H, lay ? group_size<true> : group_size<false>);
+    if (!y.P || !last_window_ok(y)) {
       delete r;
       return NTK_OK;
     }
-    y.H = y.P > 1 ? H : 0;
     y.nc = y.Wr / 16;
   }
   r->gen = !(r2::pow2_or_zero(m.ai) && r2::pow2_or_zero(m.bi) && r2::pow2_or_zero(m.ci));
@@ -675,14 +657,14 @@ int r2n_create(R2N** out, const Plan& p) {
     for (int kind = 0; kind < KINDS && ok; ++kind) {
       if ((kind == WHOLE) != (y.P == 1) || (kind == MIDDLE && y.P < 3)) continue;
       const bool cut_head = kind == MIDDLE || kind == LAST, cut_tail = kind == FIRST || kind == MIDDLE;
-      const int rows = kind == WHOLE ? n : kind == LAST ? n - (y.P - 1) * (y.Wr - 2 * y.H) : y.Wr;
+      const int rows = kind == WHOLE || kind == LAST ? y.last : y.Wr;
       Matrix q;
       q.n = rows;
       const double co[7] = {cut_head ? m.bi : m.b(0),     cut_head ? m.ci : m.c(0),     m.ai, m.bi, m.ci,
                             cut_tail ? m.ai : m.a(n - 1), cut_tail ? m.bi : m.b(n - 1)};
       q.set_reference(co);
-      std::vector<double> fl, fu, fw(std::max(rows, 0));
-      ok = rows >= 48 && rows <= y.Wr && factor_host(q, fl, fu);
+      std::vector<double> fl, fu, fw(rows);
+      ok = factor_host(q, fl, fu);
       if (!ok) break;
       for (int i = 0; i < rows; ++i) fw[i] = q.c(i) / fu[i];
       // every chunk but the first and the last has the interior's factors
