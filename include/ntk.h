@@ -210,7 +210,7 @@ typedef struct ntk_adi ntk_adi;
  *   NTK_FP64         FP64 over overlapping 32M-row windows, one warp per
  *                    window (halos exact to FP64 rounding), when N >= 128 and
  *                    the factors decay fast enough; otherwise whole systems,
- *                    several threads each, in shared memory (N >= 20), or
+ *                    several threads each, in shared memory (N >= 40), or
  *                    segmented FP64 sweeps with an N x N FP64 work array
  *                    where a system does not fit.
  *   NTK_FP32_REFINE  FP32 solve + one double-word refinement sweep per half
