@@ -201,8 +201,7 @@ template <int M, bool SCALED>
 int launch(const double* in, double* out, const AdiGeom& geo, const double* d_tab, int W, cudaStream_t st) {
   const size_t smem = smem_bytes<M>(W);
   auto kern = adi_f64_kernel<M, SCALED>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(adi_f64_kernel)");
+  if (const int rc = allow_smem(kern, smem, "cudaFuncSetAttribute(adi_f64_kernel)")) return rc;
   const long long blocks = (long long)geo.P * ((geo.ns + W - 1) / W);
   if (blocks <= 0) return NTK_OK;
   if (blocks > 0x7fffffffLL) {

@@ -170,8 +170,7 @@ int adi_launch(const double* in, double* out, const AdiGeom& geo, const RefineAr
                cudaStream_t st) {
   const size_t smem = adi_smem<M>(W, max_ncls);
   auto kern = adi_refine_kernel<M, SWEEPS, POW2, DECAY>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(adi_refine_kernel)");
+  if (const int rc = allow_smem(kern, smem, "cudaFuncSetAttribute(adi_refine_kernel)")) return rc;
   const long long blocks = (long long)geo.P * ((geo.ns + W - 1) / W);
   if (blocks <= 0) return NTK_OK;
   if (blocks > 0x7fffffffLL) {

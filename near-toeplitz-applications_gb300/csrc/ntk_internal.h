@@ -115,12 +115,16 @@ struct TablesF64 {
 void set_error(const char* fmt, ...);
 int cuda_status(cudaError_t e, const char* where);
 
-// Lets a kernel launch with smem bytes of dynamic shared memory; 48 KB need no
-// call (a call is ~1 us of a small launch's host time).
+// Lets a kernel without static shared memory launch with smem bytes of dynamic
+// shared memory; 48 KB need no call (a call is ~1 us of a small launch's host
+// time).  The limit belongs to the kernel, not to the launch: set to this
+// launch's size, another thread could lower it between this call and the
+// launch, so every caller sets the hardware's (227 KB).
+constexpr int SMEM_OPTIN = 227 * 1024;
 template <class K>
 int allow_smem(K kernel, size_t smem, const char* where) {
   if (smem <= 48 * 1024) return NTK_OK;
-  return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), where);
+  return cuda_status(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_OPTIN), where);
 }
 
 // Status bits the FP32 / FP32+refinement kernels raise in their device

@@ -192,8 +192,7 @@ int long_launch(const double* in, double* out, const LongGeom& g, const RefineAr
                 cudaStream_t st) {
   const size_t smem = long_smem(W, max_ncls);
   auto kern = long_refine_kernel<SWEEPS, POW2, DECAY, RHS>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(long_refine_kernel)");
+  if (const int rc = allow_smem(kern, smem, "cudaFuncSetAttribute(long_refine_kernel)")) return rc;
   const long long blocks = (long long)g.P * ((g.b.nsys + W - 1) / W);
   if (blocks <= 0) return NTK_OK;
   if (blocks > 0x7fffffffLL) {

@@ -507,8 +507,7 @@ int launch_x(const double* in, double* out, const Batch& b, const Args& a, int S
   }
   const size_t smem = 1024 + (size_t)S * NROWS * 8 + (size_t)2 * S * sizeof(float2) + 16;
   auto kern = r2x_kernel<RHS, SWEEPS>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(r2x_kernel)");
+  if (const int rc = allow_smem(kern, smem, "cudaFuncSetAttribute(r2x_kernel)")) return rc;
   kern<<<(unsigned)grid, 32 * S, smem, st>>>(mi, mo, a, (int)gpp);
   return cuda_status(cudaGetLastError(), "r2x_kernel");
 }

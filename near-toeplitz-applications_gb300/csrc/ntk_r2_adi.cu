@@ -293,8 +293,7 @@ namespace {
 template <class K>
 int launch_kernel(K kern, unsigned grid, unsigned block, size_t smem, cudaStream_t st, const CUtensorMap& m,
                   double* out, const AdiWin& g, const AdiKinds& ak, const char* name) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return cuda_status(e, name);
+  if (const int rc = allow_smem(kern, smem, name)) return rc;
   kern<<<grid, block, smem, st>>>(m, out, g, ak);
   return cuda_status(cudaGetLastError(), name);
 }

@@ -643,15 +643,9 @@ int launch_thomas_f64(const double* in, double* out, int n, const Batch& b, cons
   if (b.es == 1 && smem <= 200 * 1024 && (rp.kind == RHS_IDENTITY || rp.kind == RHS_COMPACT) &&
       (rp.kind == RHS_IDENTITY || n >= 4) && x_variant != 2) {
     const long long sblocks = (b.nsys + 31) / 32;
-    if (rp.kind == RHS_IDENTITY) {
-      auto k = thomas_f64_staged_kernel<RHS_IDENTITY>;
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      k<<<(unsigned)sblocks, 32, smem, stream>>>(in, out, n, b, rp, t);
-    } else {
-      auto k = thomas_f64_staged_kernel<RHS_COMPACT>;
-      cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      k<<<(unsigned)sblocks, 32, smem, stream>>>(in, out, n, b, rp, t);
-    }
+    auto k = rp.kind == RHS_IDENTITY ? thomas_f64_staged_kernel<RHS_IDENTITY> : thomas_f64_staged_kernel<RHS_COMPACT>;
+    if (const int rc = allow_smem(k, smem, "cudaFuncSetAttribute(thomas_f64_staged_kernel)")) return rc;
+    k<<<(unsigned)sblocks, 32, smem, stream>>>(in, out, n, b, rp, t);
     return cuda_status(cudaGetLastError(), "thomas_f64_staged_kernel");
   }
   if (rp.kind == RHS_IDENTITY) {

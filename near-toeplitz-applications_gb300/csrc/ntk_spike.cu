@@ -587,8 +587,7 @@ int spike_solve(SpikeSolver* s, const double* in, double* out, const Batch& b, c
   }
   const size_t smem = spike_smem(s->P);
   auto pick = [&](auto kern) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(spike_kernel)");
+    if (const int rc = allow_smem(kern, smem, "cudaFuncSetAttribute(spike_kernel)")) return rc;
     kern<<<(unsigned)b.nsys, 32 * s->P, smem, st>>>(in, out, b, s->args);
     return cuda_status(cudaGetLastError(), "spike_kernel");
   };
