@@ -31,7 +31,7 @@
 // few chunks before the pivots reach their fixed point, the interior, the
 // tail), so the factors stay in L1.
 // Measured, one thread per system against this kernel: 2046 systems of 2048
-// rows 754 -> 45 us (67 with g y on the FP64 pipe; the pipe alone: 34 us),
+// rows 754 -> 47 us (67 with g y on the FP64 pipe; the pipe alone: 34 us),
 // compact derivative of a 256 x 256 field 97 -> 8.2 us (most of it the call).
 // A system with a value that is not finite, or that overflows on the way, is
 // solved again row by row, so that inf and nan spread exactly as in the

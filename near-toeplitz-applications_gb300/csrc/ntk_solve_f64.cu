@@ -22,7 +22,7 @@
 // row loops: a condition on the row (first, last) around FP64 work becomes
 // predicated instructions there, which hold the pipe like executed ones, so
 // the end rows are handled outside (512^3 derivatives: x 1446 -> 1169 us, y
-// 1157 -> 1030 us; with g eta on the integer pipes 1143 and 833 us).  The
+// 1157 -> 1030 us; with g eta on the integer pipes 1156 and 826 us).  The
 // forward values eta are parked in the output array: many more systems are in
 // flight than the L2 holds, so the backward sweep of y and z reads them from
 // HBM (29 B per row in all) and the FP64 pipe and HBM bound one sweep each; x
