@@ -92,7 +92,8 @@ int ntk_plan_create(ntk_plan** out, int n, long long nrhs, const double coeffs[7
  *                           16-byte aligned buffers, even strides), with
  *                           strided layouts either one 16-system group per
  *                           CTA (2) or in persistent CTAs, one per SM, two
- *                           groups solved while a third loads (3); 0
+ *                           groups solved while a third loads (3, even counts of
+ *                           adjacent systems; odd ones run as 2); 0
  *                           (default) picks 3 for NTK_FP32 and 2 for
  *                           NTK_FP32_REFINE (faster on GB300); 1 the
  *                           chunked kernel above.  Other n >= 96 and

@@ -535,7 +535,11 @@ int launch_s(const double* in, double* out, const Batch& b, const Args& a, bool 
   cudaError_t e = cudaGetDevice(&dev);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return cuda_status(e, "cudaDeviceGetAttribute(SM count)");
-  if (!persistent) {
+  // A TMA store writes whole 16-byte units: with an odd number of systems the
+  // persistent kernel would overwrite the element behind the last one of a row
+  // (es is even, so there is one, outside the batch).  The other kernel stores
+  // from registers.
+  if (!persistent || (ni & 1)) {
     auto kern = r2s_kernel<RHS, SWEEPS>;
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S_SMEM);
     if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(r2s_kernel)");
