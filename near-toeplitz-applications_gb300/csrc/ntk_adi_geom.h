@@ -2,6 +2,7 @@
 // system into overlapping windows (ntk_adi_refine.cu, ntk_adi_f64.cu).
 #pragma once
 #include "ntk_internal.h"
+#include "ntk_windows.h"
 
 namespace ntk {
 
@@ -19,23 +20,8 @@ struct AdiGeom {
   long long bnd_es = 0;
 };
 
-// Window g: first row, rows written back [lo, hi), and its kind (the
-// matrix and tables it uses): 0 first, 1 middle, 2 last, 3 whole.
-struct WinRows {
-  int start, lo, hi, kind;
-};
 __host__ __device__ __forceinline__ WinRows window_rows(const AdiGeom& g, int w) {
-  WinRows r;
-  if (g.whole) {
-    r.start = 0, r.lo = 0, r.hi = g.Lw, r.kind = 3;
-  } else if (w == 0) {
-    r.start = 0, r.lo = 0, r.hi = g.L, r.kind = 0;
-  } else if (w < g.P - 1) {
-    r.start = w * g.L - g.H, r.lo = g.H, r.hi = g.H + g.L, r.kind = 1;
-  } else {
-    r.start = g.N - g.Lw, r.lo = (g.P - 1) * g.L - (g.N - g.Lw), r.hi = g.Lw, r.kind = 2;
-  }
-  return r;
+  return g.whole ? WinRows{0, 0, g.Lw, 3} : window_of(g.N, g.Lw, g.L, g.H, g.P, w);
 }
 
 }  // namespace ntk

@@ -22,6 +22,7 @@
 
 #include "ntk_long_refine.h"
 #include "ntk_refine.cuh"
+#include "ntk_windows.h"
 
 namespace ntk {
 
@@ -34,21 +35,6 @@ struct LongGeom {
   Batch b;
   int n = 0, L = 0, H = 0, P = 0;
 };
-
-struct LongWin {
-  int start, lo, hi, kind;  // first row, rows written back [lo, hi), 0 first / 1 middle / 2 last
-};
-__device__ __forceinline__ LongWin long_window(const LongGeom& g, int w) {
-  LongWin r;
-  if (w == 0) {
-    r.start = 0, r.lo = 0, r.hi = g.L, r.kind = 0;
-  } else if (w < g.P - 1) {
-    r.start = w * g.L - g.H, r.lo = g.H, r.hi = g.H + g.L, r.kind = 1;
-  } else {
-    r.start = g.n - LLW, r.lo = (g.P - 1) * g.L - (g.n - LLW), r.hi = LLW, r.kind = 2;
-  }
-  return r;
-}
 
 __host__ __device__ constexpr size_t long_smem(int W, int ncls) {
   return (((size_t)W * sys_pitch<LM>() * sizeof(double) + 2 * W * sizeof(double) + 15) & ~(size_t)15) +
@@ -114,7 +100,7 @@ __global__ void __launch_bounds__(256, RefineOcc<LM>::value)
   const int wi = (int)(blockIdx.x / nblk);
   const long long s0 = (blockIdx.x % nblk) * W;
   const int wc = (int)((g.b.nsys - s0) < W ? (g.b.nsys - s0) : W);
-  const LongWin wr = long_window(g, wi);
+  const WinRows wr = window_of(g.n, LLW, g.L, g.H, g.P, wi);
   unsigned range = 0;
 
   {

@@ -29,6 +29,7 @@
 #include "ntk_r2_adi.h"
 #include "ntk_r2_group.cuh"
 #include "ntk_r2_host.h"
+#include "ntk_windows.h"
 
 namespace ntk {
 namespace r2 {
@@ -47,15 +48,8 @@ struct AdiWin {
 };
 
 __device__ __forceinline__ void window(const AdiWin& g, int w, int& start, int& lo, int& hi, int& kind) {
-  if (g.whole) {
-    start = 0, lo = 0, hi = NROWS, kind = 3;
-  } else if (w == 0) {
-    start = 0, lo = 0, hi = g.L, kind = 0;
-  } else if (w < g.P - 1) {
-    start = w * g.L - g.H, lo = g.H, hi = g.H + g.L, kind = 1;
-  } else {
-    start = g.N - NROWS, lo = (g.P - 1) * g.L - (g.N - NROWS), hi = NROWS, kind = 2;
-  }
+  const WinRows r = g.whole ? WinRows{0, 0, NROWS, 3} : window_of(g.N, NROWS, g.L, g.H, g.P, w);
+  start = r.start, lo = r.lo, hi = r.hi, kind = r.kind;
 }
 
 template <bool GZ>
