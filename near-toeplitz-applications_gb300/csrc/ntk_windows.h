@@ -1,7 +1,7 @@
 // ntk_windows.h -- overlapping windows of one system: Lw rows each, L = Lw -
 // 2 H central ones written back, H of halo beside them (ntk_adi_refine.cu,
-// ntk_adi_f64.cu, ntk_r2_adi.cu, ntk_long_refine.cu).  Plain C++ for the host
-// too: tests/windows_check.cpp enumerates it.
+// ntk_adi_f64.cu, ntk_long_refine.cu).  Plain C++ for the host too:
+// tests/windows_check.cpp enumerates it.
 #pragma once
 
 #ifdef __CUDACC__
